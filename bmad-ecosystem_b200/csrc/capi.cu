@@ -294,6 +294,7 @@ int bmadgpu_ctx_destroy(bmadgpu_ctx* c) {
   cudaFree(c->d_tvec);
   cudaFree(c->d_tbeta);
   cudaFree(c->d_tstate);
+  cudaFree(c->d_work);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return BMADGPU_OK;

@@ -53,11 +53,48 @@ struct bmadgpu_ctx {
   int32_t* d_i32 = nullptr;       // state, ix_ele, ix_turn, location: 4 * cap
   bmadgpu_tuning tuning;
   int64_t launches = 0;           // kernel launches enqueued
+  // scratch of the calls that need some for their own duration (Workspace), kept up to kKeptWork bytes
+  void* d_work = nullptr;
+  size_t work_cap = 0;
   // autotuner trial copies
   int64_t tune_cap = 0;
   double* d_tvec = nullptr;
   double* d_tbeta = nullptr;
   int32_t* d_tstate = nullptr;
+};
+
+// Device scratch for one call on a context: the context's own block, grown as needed and kept for the
+// next call (allocating and freeing 16 bytes a particle took longer than the statistics it served), or, above kKeptWork, a block freed with this object. A context is one host thread's and
+// its work is ordered by its stream; every user waits for its stream before it returns.
+constexpr size_t kKeptWork = (size_t)128 << 20;
+struct Workspace {
+  bmadgpu_ctx* c;
+  void* ptr = nullptr;
+  bool own = false;
+  explicit Workspace(bmadgpu_ctx* ctx) : c(ctx) {}
+  Workspace(const Workspace&) = delete;
+  Workspace& operator=(const Workspace&) = delete;
+  ~Workspace() {
+    if (own) cudaFree(ptr);
+  }
+  bool get(size_t bytes) {
+    if (bytes > kKeptWork) {
+      own = cudaMalloc(&ptr, bytes) == cudaSuccess;
+      return own;
+    }
+    if (bytes > c->work_cap) {
+      cudaFree(c->d_work);
+      c->d_work = nullptr;
+      c->work_cap = 0;
+      if (cudaMalloc(&c->d_work, bytes) != cudaSuccess) {
+        c->d_work = nullptr;
+        return false;
+      }
+      c->work_cap = bytes;
+    }
+    ptr = c->d_work;
+    return true;
+  }
 };
 
 struct bmadgpu_lattice {

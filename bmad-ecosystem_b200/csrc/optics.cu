@@ -640,7 +640,7 @@ extern "C" int bmadgpu_beam_init_gaussian(bmadgpu_ctx* c, const bmadgpu_param* p
 
   // scratch: deviates of the jitters, statistics partials and sums
   void* mem = nullptr;
-  const size_t scratch = sizeof(double) * (8 + (size_t)kStatBlocks * kStatPass2 + kStatSums);
+  const size_t scratch = sizeof(double) * (8 + (size_t)kStatPartial + kStatSums);
   if (cudaMalloc(&mem, scratch) != cudaSuccess) return fail(BMADGPU_ENOMEM, "cannot allocate the beam-init scratch");
   struct Free {
     void* p;
@@ -648,7 +648,7 @@ extern "C" int bmadgpu_beam_init_gaussian(bmadgpu_ctx* c, const bmadgpu_param* p
   } freer{mem};
   double* d_extra = (double*)mem;
   double* d_partial = d_extra + 8;
-  double* d_sums = d_partial + (size_t)kStatBlocks * kStatPass2;
+  double* d_sums = d_partial + (size_t)kStatPartial;
 
   double extra[8];
   if (normals) {
