@@ -394,9 +394,9 @@ BG_HD void vjp_element(const EleHdr& h, const double* __restrict__ pool, const P
       return;
     case K_QUAD: {
       const int np = h.n_pole, n_step = h.n_step;
-      const double* kh = b + 3;
+      const double* kh = b + QD_FIXED;
       const double* kf = kh + 2 * np;
-      const double* mis = b + 3 + 4 * np;
+      const double* mis = kh + kick_doubles(np, n_step);
       const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
       const double b1 = b[0], length = b[1], sl = b[2];
       AdjTape t;
@@ -421,9 +421,9 @@ BG_HD void vjp_element(const EleHdr& h, const double* __restrict__ pool, const P
     }
     case K_THICK: {
       const int np = h.n_pole, n_step = h.n_step;
-      const double* kh = b + 1;
+      const double* kh = b + TH_FIXED;
       const double* kf = kh + 2 * np;
-      const double* mis = b + 1 + 4 * np;
+      const double* mis = kh + kick_doubles(np, n_step);
       const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
       const double sl = b[0];
       AdjTape t;

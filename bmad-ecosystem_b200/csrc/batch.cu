@@ -88,8 +88,13 @@ struct Variant {
   const void* fn;
   const void* fn_lean;
 };
+#if defined(BG_FAST_MAPS)
+#define BG_BATCH_VARIANT(B, M) \
+  {B, M, (const void*)k_batch_track<B, M, false, true>, (const void*)k_batch_track<B, M, false, true>}
+#else
 #define BG_BATCH_VARIANT(B, M) \
   {B, M, (const void*)k_batch_track<B, M, false, true>, (const void*)k_batch_track<B, M, false, false>}
+#endif
 const Variant kVariants[] = {
     BG_BATCH_VARIANT(64, 8),  BG_BATCH_VARIANT(64, 12), BG_BATCH_VARIANT(128, 3), BG_BATCH_VARIANT(128, 4),
     BG_BATCH_VARIANT(128, 5), BG_BATCH_VARIANT(128, 6), BG_BATCH_VARIANT(256, 1), BG_BATCH_VARIANT(256, 2),

@@ -38,7 +38,7 @@ __device__ __noinline__ void fma_record(const BatchVar& v, int64_t j, int32_t t_
 // REC: the instantiation for rounds that hold a frequency-map job; every other launch uses the
 // REC = false code, which has no record path at all.
 template <int BLOCK, int MINB, bool REC, bool FULL = true>
-__global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const BatchArgs a, int ppt) {
+__global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_constant__ BatchArgs a, int ppt) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ __align__(16) BatchVar sv;
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const BatchArgs a, 
       const double z_in = p.z, beta_in = p.beta;
       LossInfo li;
       if (alive) {
-        refresh(p, G);
+        refresh_particle(p, G);
         for (int turn = 0; turn < nt && alive; ++turn) {
           alive = track_turn<FULL>(p, hdr, pool, ap, G, 0, n_ele, turn == 0, turn_no0 + turn, li);
           if (REC && sv.rec && alive)

@@ -107,6 +107,8 @@ int track_device(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bunch
   a.table = lat->d_table;
   a.table_bytes = lat->pk.info.total_bytes;
   a.rare = (int32_t)lat->pk.info.rare;
+  a.ref = c->ref_forms || lat->G.hi_hot_pz == 0 ||
+          lat->pk.cold_prefix[ix_end] - lat->pk.cold_prefix[ix_start] == ix_end - ix_start;
   a.hdr_bytes = lat->pk.info.hdr_bytes;
   a.ap_bytes = lat->pk.info.ap_bytes;
   a.ix_start = ix_start;
@@ -126,6 +128,7 @@ int track_device(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bunch
   cfg.block = tu.block;
   cfg.ctas_per_sm = tu.ctas_per_sm;
   cfg.stage_smem = tu.stage_smem != 0;
+  cfg.automatic = !c->tuned;
   int cur = 0;  // which live list / count is current; live == nullptr means identity
   const int32_t* live = nullptr;
   for (int32_t done = 0; done < n_turns; done += per_launch) {
@@ -166,6 +169,10 @@ Globals make_globals(const bmadgpu_param& p) {
   g.lez_thresh = 3e-7 * p.e_tot;
   g.charge = p.charge;
   g.inv_beta0 = 1 / g.beta0;
+  uint64_t word;
+  std::memcpy(&word, &g.max_ap, sizeof(word));
+  g.hi_max_ap = g.max_ap > 0 ? (uint32_t)(word >> 32) : 0;
+  g.hi_hot_pz = 0x3fd00000u;
   return g;
 }
 
@@ -196,6 +203,7 @@ int noalloc_prepare(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bu
   a->table = lat->d_table;
   a->table_bytes = lat->pk.info.total_bytes;
   a->rare = (int32_t)lat->pk.info.rare;
+  a->ref = lat->G.hi_hot_pz == 0;
   a->hdr_bytes = lat->pk.info.hdr_bytes;
   a->ap_bytes = lat->pk.info.ap_bytes;
   a->ix_start = 0;
@@ -214,6 +222,7 @@ int noalloc_prepare(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bu
   cfg->block = c->tuning.block;
   cfg->ctas_per_sm = c->tuning.ctas_per_sm;
   cfg->stage_smem = c->tuning.stage_smem != 0;
+  cfg->automatic = !c->tuned;
   *sm_count = c->sm_count;
   *stream = c->stream;
   *launches = &c->launches;
@@ -323,6 +332,7 @@ int bmadgpu_ctx_set_tuning(bmadgpu_ctx* c, const bmadgpu_tuning* t) {
     return fail(BMADGPU_EINVAL, "block must be 64, 128, 256 or 512");
   if (t->ctas_per_sm < 0 || t->turns_per_launch < 0) return fail(BMADGPU_EINVAL, "negative tuning value");
   c->tuning = *t;
+  c->tuned = true;
   return BMADGPU_OK;
 }
 
@@ -356,6 +366,7 @@ int bmadgpu_lattice_create(bmadgpu_ctx* c, const bmadgpu_element* eles, int32_t 
   L->param = *param;
   L->eles.assign(eles, eles + n_ele);
   L->G = make_globals(*param);
+  if (L->pk.cold_prefix[n_ele] > n_ele / 2) L->G.hi_hot_pz = 0;
   cudaSetDevice(c->device);
   size_t nb = L->pk.image.size();
   if (cudaMalloc(&L->d_table, nb) != cudaSuccess ||
@@ -497,6 +508,8 @@ int bmadgpu_autotune(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_b
   t.beta = c->d_tbeta;
   t.state = c->d_tstate;
   const bmadgpu_tuning saved = c->tuning;
+  const bool was_tuned = c->tuned;
+  c->tuned = true;  // the trials' shapes are the candidates'
   struct Cand { int block, ctas, stage; };
   static const Cand cands[] = {{128, 0, 0}, {128, 4, 0}, {128, 5, 0}, {128, 6, 0}, {256, 0, 0}, {256, 2, 0},
                                {256, 3, 0}, {64, 8, 0},  {64, 12, 0}, {128, 0, 1}, {128, 4, 1}, {256, 2, 1}};
@@ -517,6 +530,7 @@ int bmadgpu_autotune(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_b
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     if (r) {
       c->tuning = saved;
+      c->tuned = was_tuned;
       return r;
     }
     CUDA_TRY(cudaEventSynchronize(e1));
@@ -528,6 +542,7 @@ int bmadgpu_autotune(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_b
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     if (r) {
       c->tuning = saved;
+      c->tuned = was_tuned;
       return r;
     }
     CUDA_TRY(cudaEventSynchronize(e1));

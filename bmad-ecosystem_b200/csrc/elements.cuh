@@ -19,9 +19,9 @@ BG_HD void body_quad(Particle& p, const EleHdr& h, const double* __restrict__ b,
   // hard/soft quadrupole fringe and the electric fringe, and with electric multipoles every
   // magnetic kick is followed by the electric one.
   const int np = h.n_pole;
-  const double* kh = b + 3;
+  const double* kh = b + QD_FIXED;
   const double* kf = kh + 2 * np;
-  const double* mis = b + 3 + 4 * np;
+  const double* mis = kh + kick_doubles(np, h.n_step);
   const bool has_t = h.flags & F_TILT;
   const double* xb = (FULL && (h.flags & F_EXTRA)) ? el : nullptr;
   const bool elec = xb && xb[0] != 0;
@@ -52,9 +52,9 @@ BG_HD void body_thick(Particle& p, const EleHdr& h, const double* __restrict__ b
                       const Globals& G) {
   // track_a_thick_multipole, bmad/low_level/track_a_thick_multipole.f90:18-133
   const int np = h.n_pole;
-  const double* kh = b + 1;
+  const double* kh = b + TH_FIXED;
   const double* kf = kh + 2 * np;
-  const double* mis = b + 1 + 4 * np;
+  const double* mis = kh + kick_doubles(np, h.n_step);
   const bool has_t = h.flags & F_TILT;
   const double* xb = (FULL && (h.flags & F_EXTRA)) ? el : nullptr;
   const bool elec = xb && xb[0] != 0;

@@ -12,6 +12,14 @@
 
 #include "../../include/bmadgpu.h"
 #include "elements.cuh"
+#if defined(BG_FAST_MAPS)
+#include "fastmaps.cuh"
+#define BG_TRACK1(p, h, pool, ap, G, first) track1_f(p, &(h), (h).fast, pool, ap, G, first)
+#define BG_REFRESH refresh_f
+#else
+#define BG_TRACK1 track1
+#define BG_REFRESH refresh
+#endif
 #include "lattice.h"
 
 using namespace bmadgpu;
@@ -39,6 +47,10 @@ Globals make_globals(const bmadgpu_param& p) {
   g.lez_thresh = 3e-7 * p.e_tot;
   g.charge = p.charge;
   g.inv_beta0 = 1 / g.beta0;
+  uint64_t word;
+  std::memcpy(&word, &g.max_ap, sizeof(word));
+  g.hi_max_ap = g.max_ap > 0 ? (uint32_t)(word >> 32) : 0;
+  g.hi_hot_pz = 0x3fd00000u;
   return g;
 }
 }  // namespace
@@ -71,11 +83,14 @@ int bmadgpu_hostcheck_track(const bmadgpu_element* eles, int32_t n_ele, const bm
     p.beta = b->beta[j];
     p.state = b->state[j];
     if (p.state != S_ALIVE) continue;
-    refresh(p, G);
+    BG_REFRESH(p, G);
+#if defined(BG_FAST_MAPS)
+    p.hot = p.hot && entry_f(p, G);
+#endif
     int lost_loc = 0, lost_ele = -1, lost_turn = -1;
     for (int turn = 0; turn < n_turns && !lost_loc; turn++) {
       for (int ie = 0; ie < n_ele; ie++) {
-        int loc = track1(p, hdr[ie], pool, ap, G, turn == 0 && ie == 0);
+        int loc = BG_TRACK1(p, hdr[ie], pool, ap, G, turn == 0 && ie == 0);
         if (loc) { lost_loc = loc; lost_ele = ie; lost_turn = turn; break; }
       }
     }

@@ -38,6 +38,10 @@ Globals host_globals(const bmadgpu_param& p) {
   g.lez_thresh = 3e-7 * p.e_tot;
   g.charge = p.charge;
   g.inv_beta0 = 1 / g.beta0;
+  uint64_t word;
+  std::memcpy(&word, &g.max_ap, sizeof(word));
+  g.hi_max_ap = g.max_ap > 0 ? (uint32_t)(word >> 32) : 0;
+  g.hi_hot_pz = 0x3fd00000u;
   return g;
 }
 

@@ -604,6 +604,165 @@ struct Packer {
   }
 };
 
+// The frame block (table.h) of a pitched misalign block (straight) or a bend frame: the position
+// transforms of offset_particle's set and unset composed into one affine map of (x, y) each.
+std::vector<double> frame_block(const std::vector<double>& mis, bool straight) {
+  typedef long double X;
+  struct Affine {
+    X a[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 0}};  // row i: coefficient of x, of y, constant
+    void add(const X* v, X sign) {
+      for (int i = 0; i < 3; i++) a[i][2] += sign * v[i];
+    }
+    void rotate(const double* w) {
+      X r[3][3];
+      for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 3; j++) r[i][j] = w[3 * i] * a[0][j] + w[3 * i + 1] * a[1][j] + w[3 * i + 2] * a[2][j];
+      std::memcpy(a, r, sizeof(r));
+    }
+  };
+  std::vector<double> out;
+  for (int side = 0; side < 2; side++) {
+    Affine A;
+    const double* w;
+    X target;
+    if (straight) {
+      const X off[3] = {mis[0], mis[1], (X)mis[4] + (side == 0 ? mis[6] : mis[5])};
+      w = &mis[side == 0 ? 9 : 18];
+      if (side == 0) {
+        A.add(off, -1);
+        A.rotate(w);
+        A.a[2][2] += mis[5];
+        target = 0;
+      } else {
+        A.a[2][2] -= mis[7];
+        A.rotate(w);
+        A.add(off, 1);
+        target = mis[8];
+      }
+    } else {
+      const int n_set = (int)mis[0], n = side == 0 ? n_set : (int)mis[1];
+      w = &mis[side == 0 ? 4 : 13];
+      for (int k = 0; k < n; k++) {
+        const double* s = &mis[BF_FIXED + BF_STEP * (k + (side == 0 ? 0 : n_set))];
+        const int op = (int)s[0];
+        const X v1[3] = {s[1], s[2], s[3]}, v2[3] = {s[13], s[14], s[15]};
+        if (op & FS_SUB) A.add(v1, -1);
+        if (op & FS_SUBZ) A.a[2][2] -= v1[2];
+        if (op & FS_MAT) A.rotate(s + 4);
+        if (op & FS_ADD) A.add(v2, 1);
+        if (op & FS_ADDZ) A.a[2][2] += v2[2];
+      }
+      target = mis[side == 0 ? 2 : 3];
+    }
+    for (int j = 0; j < 3; j++) A.a[2][j] = -A.a[2][j];
+    A.a[2][2] += target;
+    for (int i = 0; i < 3; i++)
+      for (int j = 0; j < 3; j++) out.push_back((double)A.a[i][j]);
+    out.insert(out.end(), w, w + 9);
+  }
+  return out;
+}
+
+uint32_t high_word(double v) {  // of a positive number, else 0
+  if (!(v > 0)) return 0;
+  uint64_t u;
+  std::memcpy(&u, &v, 8);
+  return (uint32_t)(u >> 32);
+}
+
+// FastHdr of a packed element: the form of fastmaps.cuh it takes, if any, and the high words below
+// which the exit coordinates are inside its aperture (r, null without one).
+FastHdr fast_header(const EleHdr& h, uint16_t flags, const std::vector<double>& blk, const ApRec* r, double max_ap) {
+  FastHdr f;
+  std::memset(&f, 0, sizeof(f));
+  f.param = h.param;
+  double x = max_ap, y = max_ap;
+  if (r && (flags & F_AP_WINDOW)) {
+    x = y = 0;
+  } else if (r && (flags & F_AP_ELLIPTICAL)) {  // the centred box with the ellipse's x/xw, y/yw below 0.7
+    x = std::min(x, 0.7 * r->x1_lim - std::fabs(r->x2_lim));
+    y = std::min(y, 0.7 * r->y1_lim - std::fabs(r->y2_lim));
+  } else if (r) {
+    auto side = [](double lo, double hi) {  // a limit of zero is none
+      return std::min(lo == 0 ? HUGE_VAL : -lo, hi == 0 ? HUGE_VAL : hi);
+    };
+    x = std::min(x, side(r->x1_lim, r->x2_lim));
+    y = std::min(y, side(r->y1_lim, r->y2_lim));
+  }
+  f.acc_x = high_word(x);
+  f.acc_y = high_word(y);
+  uint32_t c = FC_COLD;
+  if (flags & F_EXTRA) return f;
+  switch (h.kind) {
+    case K_MARKER: c = FC_MARKER; break;
+    case K_DRIFT: c = FC_DRIFT; break;
+    case K_QUAD: c = (h.n_pole == 0 && h.n_step == 1) ? FC_QUAD : FC_STEPS; break;
+    case K_THICK: {
+      const bool sext = (flags & F_KICK_B_FROM2) && h.n_pole == 3 && h.n_step == 1;
+      c = sext ? FC_SEXT : (h.n_pole == 0 && h.n_step == 1 && !(flags & F_MISALIGN)) ? FC_DRIFT : FC_STEPS;
+      break;
+    }
+    case K_SBEND: {
+      if ((flags & F_BEND_K1) || h.n_pole || h.n_step != 1) break;
+      if (flags & F_BEND_DRIFT) {
+        if (!(flags & (F_EDGE_IN | F_EDGE_OUT | F_MISALIGN))) c = FC_DRIFT;
+        break;
+      }
+      if (!(std::fabs(blk[1] * blk[0]) < 1) || !(std::fabs(blk[2] * blk[0]) < 1)) break;
+      bool upright = true;  // gt, gt2, k1_tane, fg_factor and the entrance dpx coefficient zero, gs2 = g_tot
+      for (int end = 0; end < 2; end++) {
+        const double* e = &blk[end == 0 ? SB_EDGE_IN : SB_EDGE_OUT];
+        if (!(flags & (end == 0 ? F_EDGE_IN : F_EDGE_OUT))) continue;
+        upright = upright && e[0] == 0 && e[1] == 0 && e[2] == blk[2] && e[3] == 0 && e[4] == 0 && e[5] == blk[2] &&
+                  e[6] == 0;
+        c |= end == 0 ? FC_EDGE_IN : FC_EDGE_OUT;
+      }
+      c |= FC_BEND;
+      if (blk[3] != 0) c |= FC_DG;
+      if (upright) c |= FC_UPRIGHT;
+      break;
+    }
+    default: break;
+  }
+  if (c == FC_COLD) return f;
+  if (flags & F_PITCH) c |= FC_PITCH;
+  else if (flags & F_MISALIGN) c |= FC_MISALIGN;
+  if (flags & F_TILT) c |= FC_TILT;
+  if (flags & F_AP_ENTRANCE) c |= FC_ENTRANCE;
+  f.code = c;
+  return f;
+}
+
+// The K_SBEND entries from SB_F (table.h), from extended-precision values rounded once.
+void push_bend_series(std::vector<double>& blk, double step_len, double g, double g_tot) {
+  typedef long double X;
+  const X L = step_len, a = (X)g * L, h = a / 2, s = std::sin(h), c = std::cos(h);
+  const X sinc = a == 0 ? 1 : 2 * s * c / a, cosc = a == 0 ? (X)0.5 : 2 * s * s / (a * a);
+  const X h0 = L * sinc, xi0 = L * L * (X)g * cosc, Lc2 = h0 * h0 + xi0 * xi0, Lc = std::sqrt(Lc2);
+  const X q0 = (X)g_tot * (X)g_tot * Lc2 / 4;
+  // F(q) = asin(sqrt q)/sqrt q = sum c_n q^n, c_n/c_(n-1) = (2n-1)^2 / (2n (2n+1)); its Taylor
+  // coefficients f_k = sum_n c_n binomial(n, k) q0^(n-k)
+  X f[7] = {0, 0, 0, 0, 0, 0, 0}, cn = 1;
+  X pw[7] = {1, 0, 0, 0, 0, 0, 0};  // q0^(n-k)
+  for (int n = 0; n < 400; n++) {
+    if (n > 0) {
+      cn *= (X)((2 * n - 1) * (2 * n - 1)) / (X)(2 * n * (2 * n + 1));
+      for (int k = 6; k > 0; k--) pw[k] = pw[k - 1];
+      pw[0] *= q0;
+    }
+    X bin = 1;
+    for (int k = 0; k < 7 && k <= n; k++) {
+      f[k] += cn * bin * pw[k];
+      bin = bin * (n - k) / (k + 1);
+    }
+    if (n > 6 && cn * bin * pw[6] < 1e-22L) break;  // bin: binomial(n, 7) here, above the last one used
+  }
+  blk.insert(blk.end(), {g, step_len, blk[5], blk[6], (double)h0, (double)(s / c), (double)(2 * xi0), (double)(2 * h0), (double)(1 / Lc2),
+                         (double)Lc2, (double)((X)g_tot * (X)g_tot / 4), (double)Lc});
+  for (X v : f) blk.push_back((double)v);
+  blk.push_back(g_tot == g ? 0.0 : (double)(Lc * f[0] - L));
+}
+
 void push_kicks(std::vector<double>& blk, const double* a, const double* b, int n_pole, double scale) {
   for (int n = 0; n < n_pole; n++) {
     blk.push_back(scale * b[n]);
@@ -611,15 +770,14 @@ void push_kicks(std::vector<double>& blk, const double* a, const double* b, int 
   }
 }
 
-// True if the two kick arrays starting at blk[off] (n_pole (b_n, a_n) pairs each, as the device
-// reads them) hold only normal multipoles from order 2 up: every a_n zero and b_0 = b_1 = 0.
+// True if the kick arrays starting at blk[off] (n_pole (b_n, a_n) pairs each, as the device reads
+// them, to the end of blk) hold only normal multipoles from order 2 up: every a_n zero and b_0 = b_1 = 0.
 bool kicks_b_from2(const std::vector<double>& blk, size_t off, int n_pole) {
   if (n_pole < 3) return false;
-  for (int arr = 0; arr < 2; arr++)
-    for (int n = 0; n < n_pole; n++) {
-      const double bn = blk[off + 2 * (arr * n_pole + n)], an = blk[off + 2 * (arr * n_pole + n) + 1];
-      if (an != 0 || (n < 2 && bn != 0)) return false;
-    }
+  for (size_t k = off; k + 1 < blk.size(); k += 2) {
+    const int n = (int)((k - off) / 2) % n_pole;
+    if (blk[k + 1] != 0 || (n < 2 && blk[k] != 0)) return false;
+  }
   return true;
 }
 
@@ -719,7 +877,6 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
       int key = e.key;
       if (!e.is_on && key != BMADGPU_SBEND && key != BMADGPU_MULTIPOLE && key != BMADGPU_AB_MULTIPOLE)
         key = BMADGPU_DRIFT;  // track1_bmad.f90:51-60
-      if (e.l == 0) flags |= F_ZERO_LEN;
 
       // aperture (check_aperture_limit.f90), offset_moves_aperture = F
       if (p.aperture_limit_on && e.aperture_at != BMADGPU_NO_END) {
@@ -820,14 +977,14 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
           if (ix_mag_max > -1 || ix_elec_max > -1) n_step = std::max(nint(std::fabs(e.l) / ds_step), 1);
           double r_step = 1.0 / n_step;
           double step_len = e.l * r_step;
-          blk = {b1, e.l, step_len};
+          blk = {b1, e.l, step_len, e.l == 0 ? 0.0 : b1 / e.l, e.l == 0 ? 0.0 : b1 / e.l * (step_len * step_len)};
           eblk = extra_block(e, p, ae, be, ix_elec_max, step_len / 2, step_len);
           if (ix_mag_max > -1) {
             flags |= F_KICKS;
             h.n_pole = (uint8_t)(ix_mag_max + 1);
             push_kicks(blk, a, b, ix_mag_max + 1, r_step / 2);
-            push_kicks(blk, a, b, ix_mag_max + 1, r_step);
-            if (kicks_b_from2(blk, 3, ix_mag_max + 1)) flags |= F_KICK_B_FROM2;
+            if (n_step > 1) push_kicks(blk, a, b, ix_mag_max + 1, r_step);
+            if (kicks_b_from2(blk, QD_FIXED, ix_mag_max + 1)) flags |= F_KICK_B_FROM2;
           }
           h.n_step = (uint16_t)(e.l == 0 ? 0 : n_step);
           if (has_misalign) misalign_block(tilt_tot);
@@ -852,7 +1009,7 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
                            ? 1 : std::max(nint(std::fabs(e.l / ds_step)), 1);
           double r_step = 1.0 / n_step;
           double step_len = e.l / n_step;
-          blk = {step_len};
+          blk = {step_len, 0.0};
           if (key != BMADGPU_MONITOR && key != BMADGPU_INSTRUMENT && key != BMADGPU_PIPE &&
               key != BMADGPU_RCOLLIMATOR && key != BMADGPU_ECOLLIMATOR && key != BMADGPU_KICKER &&
               key != BMADGPU_HKICKER && key != BMADGPU_VKICKER)
@@ -872,8 +1029,9 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
             flags |= F_KICKS;
             h.n_pole = (uint8_t)(ix_mag_max + 1);
             push_kicks(blk, a, b, ix_mag_max + 1, r_step / 2);
-            push_kicks(blk, a, b, ix_mag_max + 1, r_step);
-            if (kicks_b_from2(blk, 1, ix_mag_max + 1)) flags |= F_KICK_B_FROM2;
+            if (n_step > 1) push_kicks(blk, a, b, ix_mag_max + 1, r_step);
+            if (ix_mag_max >= 2) blk[1] = blk[TH_FIXED + 4];
+            if (kicks_b_from2(blk, TH_FIXED, ix_mag_max + 1)) flags |= F_KICK_B_FROM2;
           }
           h.n_step = (uint16_t)n_step;
           if (has_misalign) misalign_block(tilt_tot);
@@ -930,6 +1088,7 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
             double cdpx = gt * ge * (1 + 2 * (tan_e * tan_e));
             blk.insert(blk.end(), {gt, gt2, gs2, k1_tane, fg_factor, ge, cdpx});
           }
+          push_bend_series(blk, step_len, g, g_tot);
           if (e.fringe_type == BMADGPU_FRINGE_BASIC_BEND || e.fringe_type == BMADGPU_FRINGE_HARD_EDGE_ONLY) {
             if (e.fringe_at == BMADGPU_ENTRANCE_END || e.fringe_at == BMADGPU_BOTH_ENDS) flags |= F_EDGE_IN;
             if (e.fringe_at == BMADGPU_EXIT_END || e.fringe_at == BMADGPU_BOTH_ENDS) flags |= F_EDGE_OUT;
@@ -1010,6 +1169,10 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
       }
       h.flags = flags;
       h.param = pk.add_block(blk);
+      // a frame where there is no extra block: EleHdr::extra names it
+      if ((flags & F_PITCH) && !(flags & F_EXTRA)) h.extra = pk.add_block(frame_block(mis, h.kind != K_SBEND));
+      h.fast = fast_header(h, flags, blk, (flags & (F_AP_ENTRANCE | F_AP_EXIT)) ? &pk.ap[h.ap_index] : nullptr,
+                           p.max_aperture_limit);
       out.n_step[i] = h.n_step;
       pk.hdr.push_back(h);
     }
@@ -1032,6 +1195,9 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
     std::memcpy(out.image.data(), pk.hdr.data(), ti.hdr_bytes);
     if (ti.ap_bytes) std::memcpy(out.image.data() + ti.hdr_bytes, pk.ap.data(), ti.ap_bytes);
     std::memcpy(out.image.data() + ti.hdr_bytes + ti.ap_bytes, pk.pool.data(), pk.pool.size() * sizeof(double));
+    out.cold_prefix.assign(n_ele + 1, 0);
+    for (int i = 0; i < n_ele; i++)
+      out.cold_prefix[i + 1] = out.cold_prefix[i] + ((pk.hdr[i].fast.code & FC_BODY) == FC_COLD);
     out.ref_time_prefix.assign(n_ele + 1, 0.0);
     for (int i = 0; i < n_ele; i++) out.ref_time_prefix[i + 1] = out.ref_time_prefix[i] + eles[i].delta_ref_time;
     return BMADGPU_OK;

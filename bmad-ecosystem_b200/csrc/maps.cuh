@@ -19,6 +19,12 @@
 
 #include "table.h"
 
+// The default device build tracks with the forms of fastmaps.cuh; the correctly rounded build and
+// the host checks of bit equality with the forms of this file.
+#if defined(__CUDACC__) && !defined(BG_CR_MATH)
+#define BG_FAST_MAPS 1
+#endif
+
 // The maps' transcendentals: correctly rounded with BG_CR_MATH (device, or the test-only host
 // build made with it), otherwise the device's or host's libm.
 #if defined(BG_CR_MATH)
@@ -96,6 +102,10 @@ struct Particle {
   double e_factor;          // 1 / (1 + pz)                                                  (hwang edge)
   double lez_a;             // 1 - 3 (pz beta0**2)/2 + pz**2 f   or  beta - beta0           (low-energy dz)
   bool lez_series;          // series branch of low_energy_z_correction
+#if defined(BG_FAST_MAPS)
+  double lez;               // low_energy_z_correction per unit length
+  bool hot;                 // refresh_f
+#endif
 };
 
 BG_HD double sqrt_one(double x) {  // sim_utils/special_functions/sqrt_one.f90
@@ -140,17 +150,21 @@ BG_HD double div_rcp(double a, double b, double y) {
 #endif
 constexpr real_const kRcp6 = 1.0 / 6.0;  // RN(1/6): the divisor of the Taylor terms x/6
 
+BG_HD void refresh_lez(Particle& p, const Globals& g) {
+  // low_energy_z_correction.f90:43-52
+  double b0pz = g.beta0 * p.pz;
+  p.lez_series = g.mass * (b0pz * b0pz) < g.lez_thresh;
+  if (p.lez_series) p.lez_a = 1 - 3 * (p.pz * g.lez_b02) / 2 + (p.pz * p.pz) * g.lez_f;
+  else p.lez_a = p.beta - g.beta0;
+}
+
 BG_HD void refresh(Particle& p, const Globals& g) {
   double delta = p.pz;
   double rel_pc = 1 + delta;
   double pr = g.p0c * rel_pc;
   p.dzb = sqrt_one((g.mass2 * (2 * delta + delta * delta)) / (pr * pr + g.mass2));
   p.e_factor = 1 / (1 + p.pz);
-  // low_energy_z_correction.f90:43-52
-  double b0pz = g.beta0 * p.pz;
-  p.lez_series = g.mass * (b0pz * b0pz) < g.lez_thresh;
-  if (p.lez_series) p.lez_a = 1 - 3 * (p.pz * g.lez_b02) / 2 + (p.pz * p.pz) * g.lez_f;
-  else p.lez_a = p.beta - g.beta0;
+  refresh_lez(p, g);
 }
 
 // low_energy_z_correction, bmad/low_level/low_energy_z_correction.f90:22-57

@@ -7,6 +7,9 @@
 // lost as track1_bunch_hom leaves it (bmad/multiparticle/beam_utils.f90:81-86).
 #pragma once
 #include "elements.cuh"
+#if defined(BG_FAST_MAPS)
+#include "fastmaps.cuh"
+#endif
 
 namespace bmadgpu {
 
@@ -23,9 +26,19 @@ struct SoA {
 };
 
 __device__ __forceinline__ void load_hdr(const EleHdr* hdr, int i, EleHdr& h) {
-  uint4 raw = *reinterpret_cast<const uint4*>(hdr + i);
-  h = *reinterpret_cast<const EleHdr*>(&raw);
+  const uint4 raw = *reinterpret_cast<const uint4*>(hdr + i);  // the fields before FastHdr
+  memcpy(&h, &raw, sizeof(raw));
 }
+
+#if defined(BG_FAST_MAPS)
+__device__ __forceinline__ void load_fast(const EleHdr* hdr, int i, FastHdr& f) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(&hdr[i].fast);
+  f.code = raw.x;
+  f.param = raw.y;
+  f.acc_x = raw.z;
+  f.acc_y = raw.w;
+}
+#endif
 
 struct LossInfo {
   int loc = 0, ele = -1, turn = -1;  // coord%location, element and turn of the loss
@@ -43,11 +56,41 @@ __device__ __forceinline__ void load_particle(const SoA& s, int64_t j, Particle&
   p.state = s.state[j];
 }
 
+// The particle's cached functions of pz, as the element forms of this build read them.
+__device__ __forceinline__ void refresh_particle(Particle& p, const Globals& G) {
+#if defined(BG_FAST_MAPS)
+  refresh_f(p, G);
+#else
+  refresh(p, G);
+#endif
+}
+
 // One turn over elements [ix_start, ix_end). Returns false (and fills li) if the particle is lost.
-template <bool FULL = true>
+// FULL: see elements.cuh; the forms of fastmaps.cuh keep the rare element forms out of line, so
+// with them one instance serves. REF: the reference's forms in every build.
+template <bool FULL = true, bool REF = false>
 __device__ __forceinline__ bool track_turn(Particle& p, const EleHdr* __restrict__ hdr, const double* __restrict__ pool,
                                            const ApRec* __restrict__ ap, const Globals& G, int ix_start, int ix_end,
                                            bool first_turn, int turn_no, LossInfo& li) {
+#if defined(BG_FAST_MAPS)
+  if (!REF) {
+    if (first_turn) p.hot = p.hot && entry_f(p, G);
+    FastHdr next;  // the next element's, loaded while this one's arithmetic runs
+    load_fast(hdr, ix_start, next);
+    for (int ie = ix_start; ie < ix_end; ++ie) {
+      const FastHdr f = next;
+      load_fast(hdr, ie + 1 < ix_end ? ie + 1 : ie, next);
+      const int loc = track1_f(p, hdr + ie, f, pool, ap, G, first_turn && ie == ix_start);
+      if (loc) {
+        li.loc = loc;
+        li.ele = ie;
+        li.turn = turn_no;
+        return false;
+      }
+    }
+    return true;
+  }
+#endif
   for (int ie = ix_start; ie < ix_end; ++ie) {
     EleHdr h;
     load_hdr(hdr, ie, h);

@@ -36,7 +36,6 @@ enum Flag : uint16_t {
   F_BEND_K1 = 1 << 7,      // sbend body with k1 (sbend_body_with_k1_map)
   F_REF_ORB_N0 = 1 << 8,   // thin multipole: n = 0 as a zero-length bend (MAD convention)
   F_BEND_DRIFT = 1 << 9,   // sbend with g == 0 and dg == 0 or zero step: drift body
-  F_ZERO_LEN = 1 << 10,    // element length is zero
   F_TILT = 1 << 11,        // misalign block carries a non-zero tilt rotation
   F_KICK_B_FROM2 = 1 << 12, // both kick arrays: every a_n zero and b_0 = b_1 = 0, at least 3 orders
   F_PITCH = 1 << 13,       // misalign block of the pitched form (straight elements) or the bend frame
@@ -44,14 +43,43 @@ enum Flag : uint16_t {
   F_AP_WINDOW = 1 << 15    // the aperture record carries collimator phase-space windows
 };
 
-struct EleHdr {            // 16 bytes
+// FastHdr::code: the element's form in fastmaps.cuh and what goes with it.
+enum FastCode : uint32_t {
+  FC_COLD = 0,             // none
+  FC_MARKER = 1,
+  FC_DRIFT = 2,
+  FC_QUAD = 3,             // one step, no kicks
+  FC_SEXT = 4,             // one step, normal kicks of order 2 alone
+  FC_BEND = 5,             // one exact step
+  FC_STEPS = 6,            // quadrupole or thick multipole, any steps and kicks
+  FC_BODY = 7,
+  FC_MISALIGN = 1 << 3,    // offsets (and tilt) without pitches; ref_tilt of a bend
+  FC_TILT = 1 << 4,
+  FC_EDGE_IN = 1 << 5,     // Hwang edges
+  FC_EDGE_OUT = 1 << 6,
+  FC_UPRIGHT = 1 << 7,     // both of upright faces without fringe integral and field index
+  FC_ENTRANCE = 1 << 8,    // aperture checked at the entrance
+  FC_DG = 1 << 9,          // bend with dg
+  FC_PITCH = 1 << 10       // frame block (pitches, z_offset, misaligned bends)
+};
+
+struct FastHdr {           // 16 bytes
+  uint32_t code;
+  uint32_t param;          // EleHdr::param
+  // high words: an exit coordinate whose |value| has a smaller one is inside the element's exit
+  // aperture and max_aperture_limit; 0 where only the full test decides
+  uint32_t acc_x, acc_y;
+};
+
+struct EleHdr {            // 32 bytes
   uint8_t kind;
   uint8_t n_pole;          // number of multipole orders kicked (ix_mag_max + 1), 0 = none
   uint16_t flags;
   uint16_t n_step;
   uint16_t ap_index;       // index into the aperture records
   uint32_t param;          // offset (in doubles) of the parameter block in the pool
-  uint32_t extra;          // offset (in doubles) of the extra block (F_EXTRA), else 0
+  uint32_t extra;          // offset (in doubles) of the extra block (F_EXTRA) or the frame block (F_PITCH), else 0
+  FastHdr fast;
 };
 
 struct ApRec {             // 112 bytes
@@ -67,18 +95,23 @@ struct ApRec {             // 112 bytes
 
 // Parameter block layouts (indices in doubles from EleHdr::param).
 // K_DRIFT:  [0] L
-// K_QUAD:   [0] b1  [1] L  [2] step_len  then kicks, then misalign
-// K_THICK:  [0] step_len  then kicks, then misalign
+// K_QUAD:   [0] b1  [1] L  [2] step_len  [3] b1/L  [4] b1 step_len^2/L  then kicks, then misalign
+// K_THICK:  [0] step_len  [1] b_2 of the end kick  then kicks, then misalign
 // K_SBEND:  [0] step_len [1] g [2] g_tot [3] dg [4] angle [5] cos_a [6] sin_a [7] sinc_a
 //           [8] cosc_a [9] (g step_len)^2 sincc_a [10] k1 = b1/L [11] f_p0c = r_step p0c/(c q)
 //           [12..18] entrance edge: gt gt2 gs2 k1_tane fg_factor g_tot gt*g_tot*(1+2tan^2)
 //           [19..25] exit edge:     (same)
+//           from SB_F (bend_step_f, fastmaps.cuh): [0] g [1] step_len [2] cos_a [3] sin_a
+//           [4] h0 = step_len sinc_a  [5] tan(angle/2)  [6] 2 xi0, xi0 = step_len^2 g cosc_a  [7] 2 h0
+//           [8] 1/L_c0^2, L_c0 the chord  [9] L_c0^2  [10] g_tot^2/4  [11] L_c0  [12..18] Taylor
+//           coefficients of asin(s)/s in s^2 at q0 = (g_tot L_c0/2)^2
+//           [19] L_c0 asin(s0)/s0 - step_len (zero without dg)
 //           then kicks (bend form: plain b_n, a_n), then misalign (ref_tilt only: cos, sin)
 // K_THIN:   per order n < n_pole: [knl, cos(tilt), sin(tilt), tilt == 0], then misalign
 // K_RFCAV:  [0] voltage [1] rf_frequency [2] phi0 [3] twopi*phi0_multipass [4] slice_len
 //           [5] n_slice  then kicks (half kicks 0.5*r_step), then misalign
-// kicks: n_pole pairs for the end (half) kick followed, for K_QUAD/K_THICK, by n_pole pairs for
-//        the interior (full) kick: (b_n*scale, a_n*scale), n = 0 .. n_pole-1.
+// kicks: n_pole pairs for the end (half) kick followed, for K_QUAD/K_THICK of several steps, by
+//        n_pole pairs for the interior (full) kick: (b_n*scale, a_n*scale), n = 0 .. n_pole-1.
 // misalign: [x_off, y_off, cos_t, sin_t]; with F_PITCH (straight elements with x/y pitch or
 //           z_offset) followed by [z_off, L/2, L/2 - 0, L/2 - L, 2 (L/2)] and the rotations W^-1
 //           and W of floor_angles_to_w_mat(x_pitch, y_pitch, 0), row-major: 27 doubles
@@ -88,6 +121,9 @@ struct ApRec {             // 112 bytes
 //           acting on the position r = (x, y, 0): op & FS_SUB: r -= v1; FS_SUBZ: r_z -= v1_z;
 //           FS_MAT: r = M r; FS_ADD: r += v2; FS_ADDZ: r_z += v2_z (in that order). W rotates the
 //           momentum; the particle then drifts from r_z to s_target.
+// frame block (F_PITCH without F_EXTRA; fastmaps.cuh): for set, then unset: rows (a, b, c) of the
+//           position (x', y', ds) = a x + b y + c, ds the drift to the edge that follows, and the
+//           rotation W of the momentum, row-major: 2 x 18 doubles
 // extra block (F_EXTRA; quadrupole, sextupole, octupole, thick_multipole with electric multipoles
 //           or an edge fringe, sbend with electric multipoles or fringe_type full):
 //           [0] n_elec  [1] electric kick scale at the ends  [2] scale of the interior kicks
@@ -105,7 +141,14 @@ struct ApRec {             // 112 bytes
 //           longitudinal fringe, EX_HARD hard_multipole_edge_kick, EX_SOFT
 //           soft_quadrupole_edge_kick, EX_EXACT exact_bend_edge_kick (in place of Hwang's), EX_ESEP
 //           the elseparator's longitudinal fringe.
-constexpr int SB_EDGE_IN = 12, SB_EDGE_OUT = 19, SB_FIXED = 26;
+constexpr int SB_EDGE_IN = 12, SB_EDGE_OUT = 19, SB_F = 26, SB_FIXED = 46, QD_FIXED = 5, TH_FIXED = 2;
+#if defined(__CUDACC__)
+#define BG_TABLE_FN __host__ __device__
+#else
+#define BG_TABLE_FN
+#endif
+// doubles of the kicks of a K_QUAD or K_THICK block
+BG_TABLE_FN constexpr int kick_doubles(int n_pole, int n_step) { return (n_step > 1 ? 4 : 2) * n_pole; }
 constexpr int EL_FIXED = 32, BF_FIXED = 22, BF_STEP = 16;
 enum EdgeBit { EX_CALL = 1, EX_ELEC = 2, EX_HARD = 4, EX_SOFT = 8, EX_EXACT = 16, EX_ESEP = 32 };
 enum FrameOp { FS_SUB = 1, FS_SUBZ = 2, FS_MAT = 4, FS_ADD = 8, FS_ADDZ = 16 };
@@ -131,6 +174,10 @@ struct Globals {            // branch constants (lat_param_struct / bmad_com) an
   double lez_thresh;        // 3d-7 * e_tot
   double charge;            // charge_of(species)
   double inv_beta0;         // 1 / beta0 (rounded), the shared reciprocal of the quotients by beta0
+  uint32_t hi_max_ap;       // high word of max_ap (accepts a coordinate inside it, fastmaps.cuh)
+  // high word of 1/4: particles with a smaller |pz| take the forms of fastmaps.cuh; 0 for a lattice with
+  // more elements without a form than with one, which tracks in the reference's forms throughout
+  uint32_t hi_hot_pz;
 };
 
 

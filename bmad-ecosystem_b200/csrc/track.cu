@@ -57,29 +57,37 @@ __device__ void add_moments(const Particle& p, bool alive, double* __restrict__ 
   }
 }
 
-template <int BLOCK, int MINB, bool FULL>
-__global__ void __launch_bounds__(BLOCK, MINB) k_track(const TrackArgs a, int stage_smem) {
+// STAGED: kGlobal and kShared read the element table from there, as kernels of their own so that the
+// element loop's loads are global or shared loads, not generic ones; kEither decides at run time
+// (a.stage), for the builds whose instances take long to compile.
+enum Staging : int { kGlobal = 0, kShared = 1, kEither = 2 };
+// REF: the reference's forms in every build (TrackArgs::ref).
+template <int BLOCK, int MINB, bool FULL, int STAGED, bool REF = false>
+__global__ void __launch_bounds__(BLOCK, MINB) k_track(const __grid_constant__ TrackArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bar;
-  const uint8_t* tbl = a.table;
+  const bool stage = STAGED == kEither ? a.stage != 0 : STAGED == kShared;
   bool staged = false;
-  if (stage_smem) {
+  if (stage) {
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      stage_table_issue(smem, a.table, a.table_bytes, &bar);
-    }
+    if (threadIdx.x == 0) stage_table_issue(smem, a.table, a.table_bytes, &bar);
     const bool ok = mbar_wait_bounded(&bar, 0);
-    // Every thread must agree; a timed-out copy falls back to reading the table from global
-    // memory and raises the error flag for the host.
+    // Every thread must agree; after a time-out the threads copy the table themselves (the same
+    // bytes, should the bulk copy still land) and the error flag tells the host.
     staged = __syncthreads_and(ok);
-    if (!staged && threadIdx.x == 0) atomicOr(a.err_flag, 1);
-    if (staged) tbl = smem;
+    if (!staged) {
+      if (threadIdx.x == 0) atomicOr(a.err_flag, 1);
+      for (uint32_t i = threadIdx.x; i < a.table_bytes / 16; i += BLOCK)
+        reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(a.table)[i];
+      __syncthreads();
+    }
   }
+  const uint8_t* tbl = stage ? smem : a.table;
   const EleHdr* hdr = reinterpret_cast<const EleHdr*>(tbl);
   const ApRec* ap = reinterpret_cast<const ApRec*>(tbl + a.hdr_bytes);
   const double* pool = reinterpret_cast<const double*>(tbl + a.hdr_bytes + a.ap_bytes);
-  const Globals G = a.G;
+  const Globals& G = a.G;
   const int64_t n_work = *a.n_work;
   const double seg_ref = a.ref_prefix[a.ix_end] - a.ref_prefix[a.ix_start];
 
@@ -95,14 +103,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_track(const TrackArgs a, int st
     bool alive = valid && p.state == S_ALIVE;
     const double z_in = p.z, beta_in = p.beta;
     LossInfo li;
-    if (alive) refresh(p, G);
+    if (alive) refresh_particle(p, G);
     for (int turn = 0; turn < a.n_turns; ++turn) {
-      if (alive) alive = track_turn<FULL>(p, hdr, pool, ap, G, a.ix_start, a.ix_end, turn == 0, a.turn0 + turn, li);
+      if (alive) alive = track_turn<FULL, REF>(p, hdr, pool, ap, G, a.ix_start, a.ix_end, turn == 0, a.turn0 + turn, li);
       if (a.moments) add_moments(p, alive, a.moments + (int64_t)turn * 28);
     }
     if (valid) store_particle(soa, j, p, alive, li, z_in, beta_in, a.n_turns, a.turn0, seg_ref, a.ref_prefix, a.ix_start);
   }
-  if (stage_smem && !staged) {
+  if (stage && !staged) {
     // Let our own bulk copy drain (bounded) before the CTA's shared memory is released.
     mbar_wait_bounded(&bar, 0);
   }
@@ -188,17 +196,55 @@ cudaError_t upload_constants() {
 // thread follows: 65536 / (BLOCK * MINB), capped at 255).
 struct Variant {
   int block, minb;
-  const void* fn;       // the kernel for every element form
-  const void* fn_lean;  // the kernel for tables without rare forms (TableInfo::rare = 0)
+  const void* fn[2];       // the kernel for every element form: table in global memory, staged
+  const void* fn_lean[2];  // the kernel for tables without rare forms (TableInfo::rare = 0)
 };
-#define BG_VARIANT(B, M) {B, M, (const void*)k_track<B, M, true>, (const void*)k_track<B, M, false>}
+#if defined(BG_FAST_MAPS)
+#define BG_KERNELS(B, M) {(const void*)k_track<B, M, true, kGlobal>, (const void*)k_track<B, M, true, kShared>}
+#define BG_VARIANT(B, M) {B, M, BG_KERNELS(B, M), BG_KERNELS(B, M)}
+// For TrackArgs::ref: one warp's latency (up to four 64-thread CTAs per SM), and the whole chip.
+#define BG_REF(B, M) \
+  {B, M, {(const void*)k_track<B, M, true, kEither, true>, (const void*)k_track<B, M, true, kEither, true>}, \
+   {(const void*)k_track<B, M, false, kEither, true>, (const void*)k_track<B, M, false, kEither, true>}}
+static const Variant kRefVariants[2] = {BG_REF(64, 4), BG_REF(256, 2)};
+#undef BG_REF
+static const Variant kVariants[] = {
+    BG_VARIANT(64, 4),  BG_VARIANT(64, 8),  BG_VARIANT(64, 12), BG_VARIANT(128, 4), BG_VARIANT(128, 6),
+    BG_VARIANT(256, 1), BG_VARIANT(256, 2), BG_VARIANT(256, 3), BG_VARIANT(512, 1),
+};
+#else
+#define BG_KERNELS(B, M, FULL) {(const void*)k_track<B, M, FULL, kEither>, (const void*)k_track<B, M, FULL, kEither>}
+#define BG_VARIANT(B, M) {B, M, BG_KERNELS(B, M, true), BG_KERNELS(B, M, false)}
 static const Variant kVariants[] = {
     BG_VARIANT(64, 8),   BG_VARIANT(64, 12), BG_VARIANT(128, 3), BG_VARIANT(128, 4), BG_VARIANT(128, 5),
     BG_VARIANT(128, 6),  BG_VARIANT(256, 2), BG_VARIANT(256, 1), BG_VARIANT(256, 3), BG_VARIANT(512, 1),
 };
+#endif
+#undef BG_KERNELS
 #undef BG_VARIANT
 
-cudaError_t launch_track(const TrackArgs& a, const LaunchCfg& cfg, int sm_count, cudaStream_t stream) {
+#if defined(BG_FAST_MAPS)
+// The shape for n particles where neither the caller nor the autotuner chose one. Up to four 64-thread
+// CTAs per SM every warp has a scheduler nearly to itself and only its own latency counts: the
+// register budget without spills, and small CTAs so that all SMs get some (10,000 particles, 50-cell
+// ring: 0.16 ms a turn against 0.20 with 80 registers). A bunch that fills the chip wants the warps:
+// 24 per SM at 80 registers (1M particles, 200-cell ring: 16.4 ms a turn against 19.9 with 16 warps at
+// 128 registers and 27.2 with 8 at 255).
+static void shape_for(int64_t n, int sm_count, LaunchCfg* cfg) {
+  const int64_t row = (int64_t)64 * sm_count;  // one 64-thread CTA on every SM
+  cfg->block = n <= 8 * row ? 64 : 256;
+  cfg->ctas_per_sm = n <= 4 * row ? 4 : n <= 8 * row ? 8 : 3;
+}
+#endif
+
+cudaError_t launch_track(const TrackArgs& args_in, const LaunchCfg& cfg_in, int sm_count, cudaStream_t stream) {
+  TrackArgs a = args_in;
+  LaunchCfg cfg = cfg_in;
+#if defined(BG_FAST_MAPS)
+  if (cfg.automatic) shape_for(a.ld, sm_count, &cfg);
+  const Variant* ref = a.ref ? &kRefVariants[a.ld <= (int64_t)256 * sm_count ? 0 : 1] : nullptr;
+  if (ref) cfg.block = ref->block;
+#endif
   int stage = (cfg.stage_smem && table_fits_smem(a.table_bytes)) ? 1 : 0;
   // ctas_per_sm selects the register budget: the variant with the largest minimum CTA count
   // not above it (0: the most registers per thread)
@@ -212,35 +258,35 @@ cudaError_t launch_track(const TrackArgs& a, const LaunchCfg& cfg, int sm_count,
   if (!v)
     for (const Variant& k : kVariants)
       if (k.block == cfg.block && (!v || k.minb < v->minb)) v = &k;
+#if defined(BG_FAST_MAPS)
+  if (ref) v = ref;
+#endif
   if (!v) return cudaErrorInvalidValue;
-  const void* fn = a.rare ? v->fn : v->fn_lean;
+  const void* const* fns = a.rare ? v->fn : v->fn_lean;
   int per_sm = 0;
-  cudaError_t err;
+  cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns[0], cfg.block, 0);
+  if (err != cudaSuccess) return err;
   if (stage) {
     // Staging is taken only where it costs no residency: a table whose copy would leave room
     // for fewer CTAs per SM than the registers allow (the multipole pool of a large ring can
     // take most of the shared memory) is read through L1 instead, which measured ~2.8x faster
     // on a 176 KB table than one staged CTA per SM.
-    int plain_sm = 0;
-    if ((err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 0)) != cudaSuccess) return err;
-    if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&plain_sm, fn, cfg.block, 0)) != cudaSuccess) return err;
-    if ((err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.table_bytes)) !=
+    int staged_sm = 0;
+    if ((err = cudaFuncSetAttribute(fns[1], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.table_bytes)) !=
         cudaSuccess)
       return err;
-    if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, cfg.block, a.table_bytes)) != cudaSuccess)
+    if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&staged_sm, fns[1], cfg.block, a.table_bytes)) !=
+        cudaSuccess)
       return err;
-    if (per_sm < plain_sm) stage = 0;
+    if (staged_sm < per_sm) stage = 0;
+    else per_sm = staged_sm;
   }
-  const size_t smem = stage ? a.table_bytes : 0;
-  err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return err;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, cfg.block, smem);
-  if (err != cudaSuccess) return err;
   if (per_sm < 1) per_sm = 1;
   // Persistent grid: one full wave; every CTA strides over the particle range.
   int64_t grid = (int64_t)sm_count * per_sm;
-  void* args[] = {(void*)&a, (void*)&stage};
-  return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(cfg.block), args, smem, stream);
+  a.stage = stage;
+  void* args[] = {(void*)&a};
+  return cudaLaunchKernel(fns[stage], dim3((unsigned)grid), dim3(cfg.block), args, stage ? a.table_bytes : 0, stream);
 }
 
 cudaError_t launch_compact(const int32_t* state, const int32_t* live_in, const int64_t* n_in, int64_t n_max,

@@ -28,12 +28,17 @@ struct TrackArgs {
   Globals G;
   int32_t* err_flag;           // device: bit 0 = table staging wait timed out
   int32_t rare;                // the table has extra blocks / pitched offsets: the full kernel
+  int32_t ref;                 // the instances with the reference's element forms inline, whatever the build:
+                               // for a range without fastmaps.cuh forms, where they are faster than the
+                               // out-of-line calls (the same bits), or on request
+  int32_t stage;               // set by launch_track: the table is staged in shared memory
 };
 
 struct LaunchCfg {
   int block = 128;             // threads per CTA
   int ctas_per_sm = 0;         // 0: as many as fit (occupancy), else a cap
   bool stage_smem = true;      // stage the element table in shared memory (TMA bulk copy)
+  bool automatic = false;      // block and ctas_per_sm by launch_track's rule on the particle count
 };
 
 int table_fits_smem(uint32_t table_bytes);
