@@ -1,21 +1,33 @@
 // adjoint.cu -- d(loss)/d(element strengths) on the GPU (bmadgpu_loss_grad of include/bmadgpu.h).
 //
-// k_adjoint: one thread per particle runs adj_particle (adjoint.cuh): the forward turns with a
-// checkpoint every `every` turns, then the reverse sweep, segment by segment from the last
-// checkpoint, re-running each segment's turns and each turn's elements so every element's
-// vector-Jacobian product sees its own input. Per-particle strength derivatives accumulate in a
-// [slot][particle] buffer (each thread owns its column: no atomics).
+// A particle's turns follow one another, forward and in reverse, and a few thousand particles do not
+// fill the chip: with one thread per particle the sweep is bound by the latency of a single warp
+// (4096 particles, 451 elements, 32 turns: 158 ms). Only what is serial by nature is left that way:
+//   k_adj_forward  one thread per particle: the turns, storing the state at the start of each turn
+//                  (or, above kTurnStore, of every `every`-th, re-run by segment in reverse);
+//   k_adj_inputs   one thread per (turn, particle): re-runs the turn, storing every element's input;
+//   k_adj_turnjac  one thread per (turn, particle): the reverse sweep with the seven unit cotangents,
+//                  i.e. the turn's Jacobian J^T;
+//   k_adj_chain    one thread per particle: lambda_t = J_t^T lambda_(t+1), 49 products a turn, storing
+//                  the cotangent at the end of each turn;
+//   k_adj_grad     one thread per (turn, particle): the reverse sweep with that cotangent, writing the
+//                  strength derivatives of the turn;
+//   k_adj_collect  adds them to each particle's [slot] column, last turn first.
+// Turns go through these in chunks from the last to the first, sized by kChunkBytes. No atomics and a
+// fixed order of every sum, so the result depends neither on scheduling nor on `every` or the chunks.
 // k_adj_reduce: one CTA per slot sums the column in a fixed order (deterministic), divides by the
 // strength (scale form -> d/dk) and writes the gradient; slot n_slot sums the loss.
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
 
 #include "adjoint.cuh"
 #include "capi_internal.h"
+#include "particle.cuh"
 
 using namespace bmadgpu;
 
@@ -26,10 +38,223 @@ cudaError_t adjoint_upload_constants();
 namespace {
 
 constexpr int kAdjBlock = 64;
+constexpr size_t kTurnStore = (size_t)1 << 30;   // turn starts kept for the whole run up to this size
+constexpr size_t kChunkBytes = (size_t)2 << 30;  // element inputs, Jacobians and derivatives of a chunk of turns
 
-__global__ void __launch_bounds__(kAdjBlock) k_adjoint(const AdjArgs a) {
+struct AdjArgs {
+  const EleHdr* hdr;
+  const ApRec* ap;
+  const double* pool;
+  int32_t n_ele;
+  int64_t N;                 // particles: stride of the per-particle buffers
+  Globals G;
+  const int32_t* param_of_ele;  // [n_ele]: gradient slot of the element, -1 if none
+  int32_t n_slot;
+  double* vec;               // [6][N] in/out
+  double* beta;              // [N] in/out
+  int32_t* state;            // [N] in/out
+  double* turns;             // [rows][7][N]: states at turn starts
+  // a chunk of n_t turns: NT = n_t N threads, thread t N + j is particle j in turn row t of the chunk
+  int64_t NT;
+  double* inputs;            // [n_ele][7][NT]
+  double* jac;               // [7][7][NT]: row c, the image of unit cotangent c
+  double* lam_end;           // [7][NT]: cotangent at the end of the turn
+  double* part;              // [n_slot][NT]; null: a chunk is one turn, added to gradbuf at once
+  double* lam;               // [7][N]: cotangent at the start of the chunk's first turn
+  double* gradbuf;           // [n_slot][N]
+  double* lossbuf;           // [N]
+  double loss_scale;
+};
+
+__device__ __forceinline__ void put7(double* q, int64_t stride, const Particle& p) {
+  q[0] = p.x;
+  q[stride] = p.px;
+  q[2 * stride] = p.y;
+  q[3 * stride] = p.py;
+  q[4 * stride] = p.z;
+  q[5 * stride] = p.pz;
+  q[6 * stride] = p.beta;
+}
+__device__ __forceinline__ void get7(const double* q, int64_t stride, Particle& p) {
+  p.x = q[0];
+  p.px = q[stride];
+  p.y = q[2 * stride];
+  p.py = q[3 * stride];
+  p.z = q[4 * stride];
+  p.pz = q[5 * stride];
+  p.beta = q[6 * stride];
+  p.state = S_ALIVE;
+}
+
+// Turns [t0, t0 + n_t) of every particle that is alive, from its vec/beta (from_vec) or from turns row
+// row_in; before turn t (every `every`-th of the run) the state goes to turns row row0 + (t - t0) / every.
+// The state after the last turn returns to vec/beta/state when from_vec is set.
+__global__ void __launch_bounds__(kAdjBlock) k_adj_forward(const __grid_constant__ AdjArgs a, int t0, int n_t, int every,
+                                                           int row0, int row_in, int from_vec) {
   const int64_t j = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x;
-  if (j < a.N) adj_particle(a, j);
+  if (j >= a.N || a.state[j] != S_ALIVE) return;
+  const int64_t N = a.N;
+  Particle p;
+  if (from_vec) {
+    p.x = a.vec[j];
+    p.px = a.vec[N + j];
+    p.y = a.vec[2 * N + j];
+    p.py = a.vec[3 * N + j];
+    p.z = a.vec[4 * N + j];
+    p.pz = a.vec[5 * N + j];
+    p.beta = a.beta[j];
+    p.state = S_ALIVE;
+  } else {
+    get7(a.turns + (int64_t)row_in * 7 * N + j, N, p);
+  }
+  refresh_particle(p, a.G);
+  LossInfo li;
+  bool alive = true;
+  for (int t = 0; t < n_t && alive; ++t) {
+    if (t % every == 0) put7(a.turns + (int64_t)(row0 + t / every) * 7 * N + j, N, p);
+    alive = track_turn<false>(p, a.hdr, a.pool, a.ap, a.G, 0, a.n_ele, t0 + t == 0, t0 + t, li);
+  }
+  if (!from_vec) return;
+  a.vec[j] = p.x;
+  a.vec[N + j] = p.px;
+  a.vec[2 * N + j] = p.y;
+  a.vec[3 * N + j] = p.py;
+  a.vec[4 * N + j] = p.z;
+  a.vec[5 * N + j] = p.pz;
+  a.beta[j] = p.beta;
+  a.state[j] = p.state;
+}
+
+// Loss and its cotangent: sum over particles alive after the run of loss_scale (x^2 + y^2).
+__global__ void k_adj_loss(const __grid_constant__ AdjArgs a) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= a.N) return;
+  const bool alive = a.state[j] == S_ALIVE;  // lost particles are outside the loss
+  const double x = a.vec[j], y = a.vec[2 * a.N + j];
+  a.lossbuf[j] = alive ? a.loss_scale * (x * x + y * y) : 0.0;
+  for (int k = 0; k < 7; k++) a.lam[k * a.N + j] = 0;
+  if (alive) {
+    a.lam[j] = 2 * a.loss_scale * x;
+    a.lam[2 * a.N + j] = 2 * a.loss_scale * y;
+  }
+}
+
+// Row row0 + t of turns is the start of the chunk's turn t; first: it is the run's first turn.
+__global__ void __launch_bounds__(128) k_adj_inputs(const __grid_constant__ AdjArgs a, int row0, int first) {
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (i >= a.NT) return;
+  const int64_t t = i / a.N, j = i - t * a.N;
+  if (a.state[j] != S_ALIVE) return;
+  Particle p;
+  get7(a.turns + (row0 + t) * 7 * a.N + j, a.N, p);
+  refresh_particle(p, a.G);
+  LossInfo li;
+  for (int ie = 0; ie < a.n_ele; ++ie) {
+    put7(a.inputs + (int64_t)ie * 7 * a.NT + i, a.NT, p);
+    track_turn<false>(p, a.hdr, a.pool, a.ap, a.G, ie, ie + 1, first && t == 0 && ie == 0, 0, li);
+  }
+}
+
+// The reverse sweep of one turn over its elements, cotangents a[NC]; GRAD: derivatives to part.
+template <int NC, bool GRAD>
+__device__ __forceinline__ void turn_sweep(const AdjArgs& A, int64_t i, Adj (&a)[NC]) {
+  AdjCache k;
+  double pz = 0, beta = 0;
+  bool have = false;
+  Particle next;
+  get7(A.inputs + (int64_t)(A.n_ele - 1) * 7 * A.NT + i, A.NT, next);
+  for (int ie = A.n_ele - 1; ie >= 0; --ie) {
+    Particle p = next;
+    if (ie > 0) get7(A.inputs + (int64_t)(ie - 1) * 7 * A.NT + i, A.NT, next);  // arrives during this element
+    if (!have || p.pz != pz || p.beta != beta) {
+      refresh(p, A.G);
+      k = adj_caches(p, A.G);
+      pz = p.pz;
+      beta = p.beta;
+      have = true;
+    }
+    double gs[NC];
+#pragma unroll
+    for (int c = 0; c < NC; c++) gs[c] = 0;
+    const EleHdr& h = A.hdr[ie];
+    if (h.kind == K_RFCAV || h.n_step > 1) refresh(p, A.G);  // the bodies that are re-run on the way
+    else p.e_factor = k.ef;
+    vjp_element<NC>(h, A.pool, p, k, a, gs, A.G);
+    if (GRAD) {
+      const int slot = A.param_of_ele[ie];
+      if (slot >= 0) {
+        if (A.part) A.part[(int64_t)slot * A.NT + i] = gs[0];
+        else A.gradbuf[(int64_t)slot * A.N + i] += gs[0];
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128) k_adj_turnjac(const __grid_constant__ AdjArgs A) {
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (i >= A.NT || A.state[i % A.N] != S_ALIVE) return;
+  Adj a[7];
+#pragma unroll
+  for (int c = 0; c < 7; c++)
+    a[c] = Adj{c == 0 ? 1.0 : 0.0, c == 1 ? 1.0 : 0.0, c == 2 ? 1.0 : 0.0, c == 3 ? 1.0 : 0.0,
+               c == 4 ? 1.0 : 0.0, c == 5 ? 1.0 : 0.0, c == 6 ? 1.0 : 0.0};
+  turn_sweep<7, false>(A, i, a);
+#pragma unroll
+  for (int c = 0; c < 7; c++) {
+    double* q = A.jac + (int64_t)c * 7 * A.NT + i;
+    q[0] = a[c].x;
+    q[A.NT] = a[c].px;
+    q[2 * A.NT] = a[c].y;
+    q[3 * A.NT] = a[c].py;
+    q[4 * A.NT] = a[c].z;
+    q[5 * A.NT] = a[c].pz;
+    q[6 * A.NT] = a[c].beta;
+  }
+}
+
+__global__ void __launch_bounds__(kAdjBlock) k_adj_chain(const __grid_constant__ AdjArgs A, int n_t) {
+  const int64_t j = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x;
+  if (j >= A.N || A.state[j] != S_ALIVE) return;
+  double l[7];
+#pragma unroll
+  for (int k = 0; k < 7; k++) l[k] = A.lam[k * A.N + j];
+  for (int t = n_t - 1; t >= 0; --t) {
+    const int64_t i = t * A.N + j;
+    double m[49];
+#pragma unroll
+    for (int k = 0; k < 49; k++) m[k] = A.jac[(int64_t)k * A.NT + i];
+#pragma unroll
+    for (int k = 0; k < 7; k++) A.lam_end[k * A.NT + i] = l[k];
+    double s[7];
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+      s[k] = 0;
+#pragma unroll
+      for (int c = 0; c < 7; c++) s[k] += l[c] * m[c * 7 + k];
+    }
+#pragma unroll
+    for (int k = 0; k < 7; k++) l[k] = s[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 7; k++) A.lam[k * A.N + j] = l[k];
+}
+
+__global__ void __launch_bounds__(128) k_adj_grad(const __grid_constant__ AdjArgs A) {
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (i >= A.NT || A.state[i % A.N] != S_ALIVE) return;
+  const double* q = A.lam_end + i;
+  Adj a[1] = {Adj{q[0], q[A.NT], q[2 * A.NT], q[3 * A.NT], q[4 * A.NT], q[5 * A.NT], q[6 * A.NT]}};
+  turn_sweep<1, true>(A, i, a);
+}
+
+__global__ void __launch_bounds__(128) k_adj_collect(const __grid_constant__ AdjArgs A, int n_t, int slot0) {
+  const int64_t j = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  if (j >= A.N || A.state[j] != S_ALIVE) return;
+  const int64_t s = slot0 + blockIdx.y;
+  double g = A.gradbuf[s * A.N + j];
+#pragma unroll 8
+  for (int t = n_t - 1; t >= 0; --t) g += A.part[s * A.NT + t * A.N + j];
+  A.gradbuf[s * A.N + j] = g;
 }
 
 // Sum of row r of a [rows][N] buffer in a fixed order; one CTA of 256 threads per row.
@@ -65,19 +290,14 @@ cudaError_t adjoint_upload_constants() {
 
 namespace {
 
-// Device buffers of one call, freed on every return path.
+// Device buffers of one call, carved from one block of the context's scratch.
 struct AdjBuffers {
-  std::vector<void*> ptrs;
+  size_t used = 0;
+  unsigned char* base = nullptr;  // null while the sizes are added up
   template <class T>
-  bool get(T** p, size_t count) {
-    void* q = nullptr;
-    if (cudaMalloc(&q, count * sizeof(T) + 16) != cudaSuccess) return false;
-    ptrs.push_back(q);
-    *p = static_cast<T*>(q);
-    return true;
-  }
-  ~AdjBuffers() {
-    for (void* p : ptrs) cudaFree(p);
+  void get(T** p, size_t count) {
+    if (base) *p = reinterpret_cast<T*>(base + used);
+    used += (count * sizeof(T) + 255) & ~(size_t)255;
   }
 };
 
@@ -137,16 +357,43 @@ extern "C" int bmadgpu_loss_grad(bmadgpu_ctx* c, const bmadgpu_lattice* lat, con
   }
   CUDA_TRY(cudaSetDevice(c->device));
   const int64_t N = b->n;
-  const int32_t n_seg = (n_turns + every - 1) / every;
-  AdjBuffers buf;
-  double *d_vec, *d_beta, *d_ckpt, *d_turn, *d_ele, *d_grad, *d_loss, *d_strength, *d_out;
-  int32_t *d_state, *d_slot;
+  // Turn starts: all of them where they fit, so that nothing is run twice; else the checkpoints of the
+  // segments and, after them, the turn starts of the segment in hand.
+  const bool whole = (size_t)N * 56 * (size_t)n_turns <= kTurnStore;
+  const int32_t seg = whole ? n_turns : std::min(every, n_turns);
+  const int32_t n_seg = (n_turns + seg - 1) / seg;
   const size_t slots = (size_t)(n_param > 0 ? n_param : 1);
-  if (!buf.get(&d_vec, 6 * N) || !buf.get(&d_beta, N) || !buf.get(&d_state, N) ||
-      !buf.get(&d_ckpt, (size_t)n_seg * 7 * N) || !buf.get(&d_turn, (size_t)every * 7 * N) ||
-      !buf.get(&d_ele, (size_t)n_ele * 7 * N) || !buf.get(&d_grad, slots * N) || !buf.get(&d_loss, N) ||
-      !buf.get(&d_strength, slots) || !buf.get(&d_out, slots + 1) || !buf.get(&d_slot, (size_t)n_ele))
-    return fail(BMADGPU_ENOMEM, "cannot allocate the adjoint's device buffers");
+  const size_t per_turn = (size_t)N * 8 * ((size_t)n_ele * 7 + 49 + 7 + slots);
+  // one wave of the Jacobian kernel (256 threads per SM), whose time a part of a second wave would double
+  const size_t wave = std::max<size_t>(1, (size_t)c->sm_count * 256 / (size_t)N);
+  const int32_t chunk =
+      (int32_t)std::max<size_t>(1, std::min({kChunkBytes / per_turn, (size_t)seg, wave}));
+  const size_t CN = (size_t)chunk * N;
+  double *d_vec, *d_beta, *d_turn, *d_ele, *d_jac, *d_lam_end, *d_part, *d_lam, *d_grad, *d_loss, *d_strength, *d_out;
+  int32_t *d_state, *d_slot;
+  Workspace work(c);
+  AdjBuffers buf;
+  for (int pass = 0; pass < 2; pass++) {
+    buf.get(&d_vec, 6 * N);
+    buf.get(&d_beta, N);
+    buf.get(&d_state, N);
+    buf.get(&d_turn, (size_t)(whole ? seg : n_seg + seg) * 7 * N);
+    buf.get(&d_ele, (size_t)n_ele * 7 * CN);
+    buf.get(&d_jac, 49 * CN);
+    buf.get(&d_lam_end, 7 * CN);
+    buf.get(&d_part, chunk > 1 ? slots * CN : 1);
+    buf.get(&d_lam, 7 * (size_t)N);
+    buf.get(&d_grad, slots * N);
+    buf.get(&d_loss, N);
+    buf.get(&d_strength, slots);
+    buf.get(&d_out, slots + 1);
+    buf.get(&d_slot, (size_t)n_ele);
+    if (pass == 0) {
+      if (!work.get(buf.used)) return fail(BMADGPU_ENOMEM, "cannot allocate the adjoint's device buffers");
+      buf.base = static_cast<unsigned char*>(work.ptr);
+      buf.used = 0;
+    }
+  }
   cudaStream_t s = c->stream;
   CUDA_TRY(cudaMemcpyAsync(d_vec, b->vec, 6 * N * sizeof(double), cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(d_beta, b->beta, N * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -161,26 +408,54 @@ extern "C" int bmadgpu_loss_grad(bmadgpu_ctx* c, const bmadgpu_lattice* lat, con
   a.ap = reinterpret_cast<const ApRec*>(lat->d_table + lat->pk.info.hdr_bytes);
   a.pool = reinterpret_cast<const double*>(lat->d_table + lat->pk.info.hdr_bytes + lat->pk.info.ap_bytes);
   a.n_ele = n_ele;
-  a.n_turns = n_turns;
-  a.every = every;
   a.N = N;
   a.G = lat->G;
   a.param_of_ele = d_slot;
-  a.ckpt = d_ckpt;
-  a.turnbuf = d_turn;
-  a.elebuf = d_ele;
-  a.gradbuf = d_grad;
-  a.lossbuf = d_loss;
+  a.n_slot = n_param;
   a.vec = d_vec;
   a.beta = d_beta;
   a.state = d_state;
+  a.turns = d_turn;
+  a.inputs = d_ele;
+  a.jac = d_jac;
+  a.lam_end = d_lam_end;
+  a.part = chunk > 1 ? d_part : nullptr;
+  a.lam = d_lam;
+  a.gradbuf = d_grad;
+  a.lossbuf = d_loss;
   a.loss_scale = 1.0 / (double)N;
   const unsigned grid = (unsigned)((N + kAdjBlock - 1) / kAdjBlock);
-  k_adjoint<<<grid, kAdjBlock, 0, s>>>(a);
+  k_adj_forward<<<grid, kAdjBlock, 0, s>>>(a, 0, n_turns, whole ? 1 : seg, 0, 0, 1);
+  k_adj_loss<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(a);
+  c->launches += 2;
+  for (int32_t g = n_seg - 1; g >= 0; --g) {
+    const int32_t t0 = g * seg, nt = std::min(seg, n_turns - t0);
+    const int32_t row0 = whole ? 0 : n_seg;
+    if (!whole) {
+      k_adj_forward<<<grid, kAdjBlock, 0, s>>>(a, t0, nt, 1, row0, g, 0);
+      c->launches++;
+    }
+    for (int32_t end = nt; end > 0;) {
+      const int32_t begin = std::max(0, end - chunk), n = end - begin;
+      a.NT = (int64_t)n * N;
+      const unsigned wide = (unsigned)((a.NT + 127) / 128);
+      k_adj_inputs<<<wide, 128, 0, s>>>(a, row0 + begin, t0 + begin == 0);
+      k_adj_turnjac<<<wide, 128, 0, s>>>(a);
+      k_adj_chain<<<grid, kAdjBlock, 0, s>>>(a, n);
+      k_adj_grad<<<wide, 128, 0, s>>>(a);
+      c->launches += 4;
+      for (int32_t s0 = 0; a.part && s0 < n_param; s0 += 32768) {
+        const dim3 all((unsigned)((N + 127) / 128), (unsigned)std::min(n_param - s0, 32768));
+        k_adj_collect<<<all, 128, 0, s>>>(a, n, s0);
+        c->launches++;
+      }
+      end = begin;
+    }
+  }
   CUDA_TRY(cudaGetLastError());
   k_adj_reduce<<<(unsigned)(n_param + 1), 256, 0, s>>>(d_grad, d_loss, N, n_param, d_strength, d_out);
   CUDA_TRY(cudaGetLastError());
-  c->launches += 2;
+  c->launches++;
   std::vector<double> out(n_param + 1);
   CUDA_TRY(cudaMemcpyAsync(out.data(), d_out, (n_param + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));

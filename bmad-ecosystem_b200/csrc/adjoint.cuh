@@ -25,288 +25,276 @@ struct Adj {
 // Elements with more body steps (or RF slices) than this are outside the adjoint path.
 constexpr int kAdjMaxSteps = 16;
 
-// d(dzb)/d(pz): dzb = beta(pz)/beta0 - 1, dbeta/dpz = p0c m^2 / E^3.
-BG_HD double d_dzb(double pz, const Globals& G) {
-  double P = G.p0c * (1 + pz);
-  double E2 = P * P + G.mass2;
-  double E = sqrt(E2);
-  return G.p0c * G.mass2 / (G.beta0 * E2 * E);
+// Functions of pz (and beta) the derivatives share: they change only at an energy kick, so a sweep over
+// the elements forms them once per stretch (adj_caches).
+struct AdjCache {
+  double ef;      // 1 / (1 + pz)
+  double ddzb;    // d(dzb)/d(pz): dzb = beta(pz)/beta0 - 1, dbeta/dpz = p0c m^2 / E^3
+  double lez_pz;  // d(low_energy_z)/d(pz) per unit length (series branch)
+  double lez_b;   // d(low_energy_z)/d(beta) per unit length (the other branch)
+};
+
+// p: caches refreshed (refresh()).
+BG_HD AdjCache adj_caches(const Particle& p, const Globals& G) {
+  AdjCache c;
+  c.ef = 1 / (1 + p.pz);
+  const double P = G.p0c * (1 + p.pz);
+  const double E2 = P * P + G.mass2;
+  c.ddzb = p.beta > 0 ? G.p0c * G.mass2 / (G.beta0 * E2 * sqrt(E2)) : 0.0;
+  if (p.lez_series) {
+    const double dlez = -3 * G.lez_b02 / 2 + 2 * p.pz * G.lez_f;
+    c.lez_pz = G.lez_me2 * (p.lez_a + p.pz * dlez);
+    c.lez_b = 0;
+  } else {
+    c.lez_pz = 0;
+    c.lez_b = 1 / G.beta0;
+  }
+  return c;
 }
 
-// z += low_energy_z(p, ds): cotangents to pz (series branch) or beta.
-BG_HD void vjp_lez(const Particle& p, double ds, Adj& a, const Globals& G) {
-  if (p.lez_series) {
-    double dlez = -3 * G.lez_b02 / 2 + 2 * p.pz * G.lez_f;
-    a.pz += a.z * ds * G.lez_me2 * (p.lez_a + p.pz * dlez);
-  } else {
-    a.beta += a.z * ds / G.beta0;
-  }
-}
+// Each primitive below forms the coefficients of its Jacobian at the input particle once and applies
+// the transpose to NC cotangents: one in the gradient sweep, seven (the unit vectors) where a whole
+// turn's Jacobian is wanted.
 
 // track_a_drift
-BG_HD void vjp_drift(const Particle& p, double L, Adj& a, const Globals& G) {
+template <int NC>
+BG_HD void vjp_drift(const Particle& p, const AdjCache& k, double L, Adj (&a)[NC]) {
   if (L == 0) return;
-  double rel = 1 + p.pz;
-  double ar = p.px / rel, br = p.py / rel;
-  double s2 = ar * ar + br * br;
-  double ps = sqrt(1 - s2);
-  double ips = 1 / ps, ips3 = ips * ips * ips;
-  double abar = a.x * L * (ips + ar * ar * ips3) + a.y * L * (ar * br * ips3) - a.z * L * ar * ips3;
-  double bbar = a.x * L * (ar * br * ips3) + a.y * L * (ips + br * br * ips3) - a.z * L * br * ips3;
-  a.px += abar / rel;
-  a.py += bbar / rel;
-  a.pz += -(abar * ar + bbar * br) / rel;
-  if (p.beta > 0) a.pz += a.z * L * d_dzb(p.pz, G);
-}
-
-// Derivatives of quad_mat2_calc's cx, sx with respect to k (quad_mat2_calc.f90:34-47).
-BG_HD void quad_cs_dk(double k, double l, double cx, double sx, double& dcx, double& dsx) {
-  double skl = sqrt(fabs(k)) * l;
-  dcx = l * sx / 2;
-  if (fabs(skl) < 1e-10) {
-    dcx = l * l / 2;
-    dsx = l * l * l / 6;
-    return;
-  }
-  double u = k * l * l;
-  if (fabs(u) < 0.1) {
-    // l^3 sum_{n>=1} n u^(n-1) / (2n+1)!, to u^4
-    dsx = l * l * l * (1.0 / 6 + u * (2.0 / 120 + u * (3.0 / 5040 + u * (4.0 / 362880 + u * (5.0 / 39916800)))));
-  } else {
-    dsx = (l * cx - sx) / (2 * k);
+  const double ar = p.px * k.ef, br = p.py * k.ef;
+  const double s2 = ar * ar + br * br;
+  const double ips = 1 / sqrt(1 - s2), l = L * ips, l3 = l * ips * ips;
+  const double xx = l + ar * ar * l3, xy = ar * br * l3, yy = l + br * br * l3, xz = ar * l3, yz = br * l3;
+  const double zb = L * k.ddzb;
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    const double ab = (a[c].x * xx + a[c].y * xy - a[c].z * xz) * k.ef;
+    const double bb = (a[c].x * xy + a[c].y * yy - a[c].z * yz) * k.ef;
+    a[c].px += ab;
+    a[c].py += bb;
+    a[c].pz += a[c].z * zb - (ab * ar + bb * br);
   }
 }
 
-// Cotangent of (k, rel) from the cotangents of one plane's quad_mat2 outputs.
-// lc: cotangent of cx (m11 and m22), l12, l21, lz0, lz1, lz2.
-BG_HD void quad_mat2_vjp(double k, double l, double rel, double lc, double l12, double l21, double lz0, double lz1,
-                         double lz2, double& gk, double& grel) {
-  double sk = sqrt(fabs(k)), skl = sk * l;
-  double cx, sx;
-  if (fabs(skl) < 1e-10) {
-    double k_l2 = k * (l * l);
-    cx = 1 + k_l2 / 2;
-    sx = (1 + k_l2 / 6) * l;
-  } else if (k < 0) {
-    cx = cos(skl);
-    sx = sin(skl) / sk;
-  } else {
-    cx = cosh(skl);
-    sx = sinh(skl) / sk;
-  }
-  double dcx, dsx;
-  quad_cs_dk(k, l, cx, sx, dcx, dsx);
-  // m12 = sx/rel, m21 = k sx rel, z0 = k(l - cx sx)/4, z1 = -k sx^2/(2 rel), z2 = -(cx sx + l)/(4 rel^2)
-  double d_cs = dcx * sx + cx * dsx;
-  gk = lc * dcx + l12 * dsx / rel + l21 * (sx + k * dsx) * rel + lz0 * ((l - cx * sx) / 4 - k * d_cs / 4) +
-       lz1 * (-(sx * sx + 2 * k * sx * dsx) / (2 * rel)) + lz2 * (-d_cs / (4 * rel * rel));
-  grel = l12 * (-sx / (rel * rel)) + l21 * k * sx + lz1 * (k * sx * sx / (2 * rel * rel)) +
-         lz2 * ((cx * sx + l) / (2 * rel * rel * rel));
-}
-
-// One quad body step (quad_step); gb1 += d/d(b1) contribution times b1 (scale form).
-BG_HD void vjp_quad_step(const Particle& p, double b1, double length, double sl, Adj& a, double& gscale,
-                         const Globals& G) {
-  double rel = 1 + p.pz;
-  double k1 = b1 / (length * rel);
-  double ax, bx, cx_, dx, zx0, zx1, zx2, ay, by, cy, dy, zy0, zy1, zy2;
-  const double ef = 1 / rel;
-  quad_mat2(-k1, sl, rel, ef, ax, bx, cx_, dx, zx0, zx1, zx2);
-  quad_mat2(k1, sl, rel, ef, ay, by, cy, dy, zy0, zy1, zy2);
-  double x = p.x, px = p.px, y = p.y, py = p.py;
-  // low_energy_z on the stepped particle: pz and beta are unchanged by the step
-  vjp_lez(p, sl, a, G);
-  Adj o = a;
-  a.x = o.x * ax + o.px * cx_ + o.z * (2 * zx0 * x + zx1 * px);
-  a.px = o.x * bx + o.px * dx + o.z * (zx1 * x + 2 * zx2 * px);
-  a.y = o.y * ay + o.py * cy + o.z * (2 * zy0 * y + zy1 * py);
-  a.py = o.y * by + o.py * dy + o.z * (zy1 * y + 2 * zy2 * py);
-  // coefficient cotangents (m11 = m22 = c)
-  double gkx, grx, gky, gry;
-  quad_mat2_vjp(-k1, sl, rel, o.x * x + o.px * px, o.x * px, o.px * x, o.z * x * x, o.z * x * px, o.z * px * px, gkx,
-                grx);
-  quad_mat2_vjp(k1, sl, rel, o.y * y + o.py * py, o.y * py, o.py * y, o.z * y * y, o.z * y * py, o.z * py * py, gky,
-                gry);
-  double gk1 = -gkx + gky;
-  double grel = grx + gry + gk1 * (-k1 / rel);
-  a.pz += grel;
-  gscale += gk1 * k1;  // k1 is proportional to b1: b1 dL/db1 = k1 dL/dk1
-}
-
-// ab_multipole_kicks with pre-scaled coefficients c = (b_n, a_n): px += kx, py += ky.
-BG_HD void vjp_ab_kicks(const Particle& p, const double* __restrict__ c, int n_pole, Adj& a, double& gscale) {
-  const double x = p.x, y = p.y;
-  double kx = 0, ky = 0, kxx = 0, kxy = 0, kyx = 0, kyy = 0;
-  for (int n = 0; n < n_pole; n++) {
-    const double b = c[2 * n], aa = c[2 * n + 1];
-    if (b == 0 && aa == 0) continue;
-    for (int m = 0; m <= n; m++) {
-      double cm = BG_CMULTI(n, m);
-      double f = cm * mexp(x, n - m) * mexp(y, m);
-      double fx = (n - m > 0) ? cm * (n - m) * mexp(x, n - m - 1) * mexp(y, m) : 0.0;
-      double fy = (m > 0) ? cm * m * mexp(x, n - m) * mexp(y, m - 1) : 0.0;
-      double cxk, cyk;  // coefficient of f in kx and ky
-      if (m % 2 == 0) {
-        cxk = b;
-        cyk = -aa;
-      } else {
-        cxk = aa;
-        cyk = b;
+// cos, sin / sqrt(k) of quad_mat2_calc (quad_mat2_calc.f90:34-47) for +-k and their derivatives with
+// respect to k. For |k| l^2 < 1/2 by the series in u = k l^2: c(u) = sum (-u)^n/(2n)!,
+// s(u) = l sum (-u)^n/(2n+1)! for the focusing sign, u -> -u for the other.
+struct QuadCs {
+  double c, s, dc, ds;
+};
+BG_HD QuadCs quad_cs(double k, double l) {  // c'' = k c: k > 0 hyperbolic
+  QuadCs q;
+  const double u = k * (l * l), l2 = l * l;
+  if (fabs(u) < 0.5) {
+    double c = 1.0 / 20922789888000.0, s = 1.0 / 355687428096000.0, dc = 8.0 / 20922789888000.0,
+           ds = 8.0 / 355687428096000.0;
+    const double f[8] = {1.0, 0.5, 1.0 / 24.0, 1.0 / 720.0, 1.0 / 40320.0, 1.0 / 3628800.0, 1.0 / 479001600.0,
+                         1.0 / 87178291200.0};
+    const double g[8] = {1.0, 1.0 / 6.0, 1.0 / 120.0, 1.0 / 5040.0, 1.0 / 362880.0, 1.0 / 39916800.0,
+                         1.0 / 6227020800.0, 1.0 / 1307674368000.0};
+#pragma unroll
+    for (int n = 7; n >= 0; n--) {
+      c = c * u + f[n];
+      s = s * u + g[n];
+      if (n > 0) {
+        dc = dc * u + n * f[n];
+        ds = ds * u + n * g[n];
       }
-      kx += cxk * f;
-      ky += cyk * f;
-      kxx += cxk * fx;
-      kxy += cxk * fy;
-      kyx += cyk * fx;
-      kyy += cyk * fy;
     }
+    q.c = c;
+    q.s = s * l;
+    q.dc = dc * l2;
+    q.ds = ds * l2 * l;
+    return q;
   }
-  gscale += a.px * kx + a.py * ky;
-  a.x += a.px * kxx + a.py * kyx;
-  a.y += a.px * kxy + a.py * kyy;
+  const double sk = sqrt(fabs(k)), skl = sk * l;
+  if (k < 0) {
+    q.c = cos(skl);
+    q.s = sin(skl) / sk;
+  } else {
+    q.c = cosh(skl);
+    q.s = sinh(skl) / sk;
+  }
+  q.dc = l * q.s / 2;
+  q.ds = (l * q.c - q.s) / (2 * k);
+  return q;
+}
+
+// One plane of a quadrupole step with k (quad_mat2_calc's), at (x, px): cotangents of k and rel as
+// coefficients of the cotangents of the plane's x', px' and of z'.
+struct QuadPlane {
+  double m11, m12, m21;      // m22 = m11
+  double zx, zp;             // dz/dx, dz/dpx
+  double kx, kp, kz;         // d/dk of x', px', z'
+  double rx, rp, rz;         // d/drel of the same
+};
+BG_HD QuadPlane quad_plane(double k, double l, double rel, double ef, double x, double px) {
+  const QuadCs q = quad_cs(k, l);
+  QuadPlane o;
+  o.m11 = q.c;
+  o.m12 = q.s * ef;
+  o.m21 = k * q.s * rel;
+  const double cs = q.c * q.s, dcs = q.dc * q.s + q.c * q.ds, s2 = q.s * q.s;
+  const double z0 = k * (l - cs) / 4, z1 = -k * s2 * ef / 2, z2 = -(cs + l) * ef * ef / 4;
+  o.zx = 2 * z0 * x + z1 * px;
+  o.zp = z1 * x + 2 * z2 * px;
+  o.kx = x * q.dc + px * q.ds * ef;
+  o.kp = px * q.dc + x * (q.s + k * q.ds) * rel;
+  o.kz = x * x * ((l - cs) / 4 - k * dcs / 4) - x * px * (s2 + 2 * k * q.s * q.ds) * ef / 2 -
+         px * px * dcs * ef * ef / 4;
+  o.rx = -px * q.s * ef * ef;
+  o.rp = x * k * q.s;
+  o.rz = -(x * px * z1 + 2 * px * px * z2) * ef;
+  return o;
+}
+
+// One quad body step (quad_step); gscale += d/d(b1) contribution times b1 (scale form).
+template <int NC>
+BG_HD void vjp_quad_step(const Particle& p, const AdjCache& k, double b1, double length, double sl, Adj (&a)[NC],
+                         double (&gscale)[NC]) {
+  const double rel = 1 + p.pz;
+  const double k1 = b1 / length * k.ef;
+  const QuadPlane X = quad_plane(-k1, sl, rel, k.ef, p.x, p.px), Y = quad_plane(k1, sl, rel, k.ef, p.y, p.py);
+  const double lp = sl * k.lez_pz, lb = sl * k.lez_b;
+#pragma unroll
+  for (int c = 0; c < NC; c++) {
+    const Adj o = a[c];
+    const double gk1 = (o.y * Y.kx + o.py * Y.kp + o.z * Y.kz) - (o.x * X.kx + o.px * X.kp + o.z * X.kz);
+    const double gr = (o.x * X.rx + o.px * X.rp + o.z * X.rz) + (o.y * Y.rx + o.py * Y.rp + o.z * Y.rz);
+    a[c].x = o.x * X.m11 + o.px * X.m21 + o.z * X.zx;
+    a[c].px = o.x * X.m12 + o.px * X.m11 + o.z * X.zp;
+    a[c].y = o.y * Y.m11 + o.py * Y.m21 + o.z * Y.zx;
+    a[c].py = o.y * Y.m12 + o.py * Y.m11 + o.z * Y.zp;
+    a[c].pz += gr - gk1 * k1 * k.ef + o.z * lp;
+    a[c].beta += o.z * lb;
+    gscale[c] += gk1 * k1;  // k1 is proportional to b1: b1 dL/db1 = k1 dL/dk1
+  }
+}
+
+// ab_multipole_kicks with pre-scaled coefficients c = (b_n, a_n): px += kx, py += ky with
+// kx - i ky = -S, S = sum (b_n + i a_n)(x + i y)^n, by Horner with its derivative.
+template <int NC>
+BG_HD void vjp_ab_kicks(const Particle& p, const double* __restrict__ c, int n_pole, Adj (&a)[NC],
+                        double (&gscale)[NC]) {
+  const double x = p.x, y = p.y;
+  double re = 0, im = 0, dr = 0, di = 0;
+  for (int n = n_pole - 1; n >= 0; n--) {
+    const double td = dr * x - di * y + re;
+    di = dr * y + di * x + im;
+    dr = td;
+    const double t = re * x - im * y + c[2 * n];
+    im = re * y + im * x + c[2 * n + 1];
+    re = t;
+  }
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    gscale[i] += a[i].py * im - a[i].px * re;
+    const double gx = a[i].py * di - a[i].px * dr, gy = a[i].px * di + a[i].py * dr;
+    a[i].x += gx;
+    a[i].y += gy;
+  }
 }
 
 // tilt (rotation by (c, s)); the inverse rotation passes -s.
-BG_HD void vjp_tilt(double c, double s, Adj& a) {
-  double ax = a.x, ay = a.y, apx = a.px, apy = a.py;
-  a.x = c * ax - s * ay;
-  a.y = s * ax + c * ay;
-  a.px = c * apx - s * apy;
-  a.py = s * apx + c * apy;
+template <int NC>
+BG_HD void vjp_tilt(double c, double s, Adj (&a)[NC]) {
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    const double ax = a[i].x, ay = a[i].y, apx = a[i].px, apy = a[i].py;
+    a[i].x = c * ax - s * ay;
+    a[i].y = s * ax + c * ay;
+    a[i].px = c * apx - s * apy;
+    a[i].py = s * apx + c * apy;
+  }
 }
 
-// Exact sbend body step (bend_exact_step).
-BG_HD void vjp_bend_exact(const Particle& p, const double* __restrict__ b, Adj& a, const Globals& G) {
-  double l = b[0], g = b[1], g_tot = b[2], dg = b[3], angle = b[4];
-  double cos_a = b[5], sin_a = b[6], sinc_a = b[7], cosc_a = b[8], gl2_sincc = b[9];
-  double x = p.x, px = p.px, py = p.py, pz = p.pz;
-  double rel = 1 + pz;
+// Exact sbend body step (bend_exact_step). In the momentum components of the rotated axes (Sp, Cp) and
+// the exit components (pxf, R) the map has no trigonometric function of the particle but the arc over
+// its chord, L_p = L_c F(q), F = asin(s)/s, q = s^2 = (g_tot L_c / 2 pt)^2:
+//   pxf = ca px + sa ps - g_tot h, h = (1 + g x) L sinc, xi = h (2 pxf + g_tot h) / (R + Cp),
+//   x' = x ca + xi - const, y' = y + py L_p / pt, z' = z + beta L / beta0 - rel L_p / pt.
+// Four directions (x, px, py, rel) are differentiated through it.
+template <int NC>
+BG_HD void vjp_bend_exact(const Particle& p, const AdjCache& k, const double* __restrict__ b, Adj (&a)[NC],
+                          const Globals& G) {
+  const double l = b[0], g = b[1], g_tot = b[2], dg = b[3];
+  const double ca = b[5], sa = b[6], sinc_a = b[7], cosc_a = b[8], gl2_sincc = b[9];
+  const double x = p.x, px = p.px, py = p.py, pz = p.pz;
+  const double rel = 1 + pz;
   if (dg == 0 && fabs(x * g) < 1e-9 && fabs(px) < 1e-9 && fabs(py) < 1e-9 && fabs(pz) < 1e-9) {
-    double rpp = rel * G.p0c;
-    double den = rpp * rpp + G.mass2;
-    double gam2 = G.mass2 / den;
-    double m56 = l * (gam2 - gl2_sincc);
-    double dm56 = l * (-G.mass2 * 2 * rpp * G.p0c / (den * den));
-    Adj o = a;
-    a.x = o.x * cos_a + o.px * (-g * sin_a) + o.z * (-g * l * sinc_a);
-    a.px = o.x * l * sinc_a + o.px * cos_a + o.z * (-g * l * l * cosc_a);
-    a.py = o.py + o.y * l;
-    a.pz = o.pz + o.x * g * l * l * cosc_a + o.px * g * l * sinc_a + o.z * (m56 + dm56 * pz);
+    const double rpp = rel * G.p0c;
+    const double den = rpp * rpp + G.mass2;
+    const double gam2 = G.mass2 / den;
+    const double m56 = l * (gam2 - gl2_sincc);
+    const double dm56 = l * (-G.mass2 * 2 * rpp * G.p0c / (den * den));
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+      const Adj o = a[i];
+      a[i].x = o.x * ca + o.px * (-g * sa) + o.z * (-g * l * sinc_a);
+      a[i].px = o.x * l * sinc_a + o.px * ca + o.z * (-g * l * l * cosc_a);
+      a[i].py = o.py + o.y * l;
+      a[i].pz = o.pz + o.x * g * l * l * cosc_a + o.px * g * l * sinc_a + o.z * (m56 + dm56 * pz);
+    }
     return;
   }
-  // forward intermediates
-  double pt = sqrt(rel * rel - py * py);
-  double g_p = g_tot / pt;
-  double u = px / pt;
-  double phi_1 = asin(u);
-  double cp = cos(angle + phi_1), sp = sin(angle + phi_1);
-  double gx1 = 1 + g * x;
-  double ls = gx1 * l * sinc_a;
-  double alpha = 2 * gx1 * sp * l * sinc_a - g_p * (ls * ls);
-  double r = cp * cp + g_p * alpha;
-  double rad = sqrt(r);
-  double xi, den = 0;
-  if (cp > 0) {
-    den = rad + cp;
-    xi = alpha / den;
+  const double pt2 = rel * rel - py * py;
+  const double ps = sqrt(pt2 - px * px), ips = 1 / ps;
+  const double ipt = 1 / sqrt(pt2);
+  const double h0 = l * sinc_a, h = h0 * (1 + g * x);
+  const double pxf = ca * px + sa * ps - g_tot * h;
+  const double R = sqrt(pt2 - pxf * pxf), iR = 1 / R;
+  const double Cp = ca * ps - sa * px;
+  const double N = 2 * pxf + g_tot * h;
+  const bool fwd = Cp > 0;
+  const double iD = fwd ? 1 / (R + Cp) : 1 / g_tot;
+  const double xi = fwd ? h * N * iD : (R - Cp) * iD;
+  const double Lv = h0 + x * sa;
+  const double Lc = sqrt(xi * xi + Lv * Lv), iLc = 1 / Lc;
+  const double s = 0.5 * g_tot * Lc * ipt, q = s * s;
+  double F, dF;  // F and dF/dq
+  if (q < 0.0078125) {
+    F = 1 + q * (1.0 / 6 + q * (3.0 / 40 + q * (5.0 / 112 + q * (35.0 / 1152 + q * (63.0 / 2816 +
+            q * (231.0 / 13312 + q * (143.0 / 10240)))))));
+    dF = 1.0 / 6 + q * (3.0 / 20 + q * (15.0 / 112 + q * (35.0 / 288 + q * (315.0 / 2816 + q * (693.0 / 6656 +
+            q * (1001.0 / 10240))))));
   } else {
-    xi = (rad - cp) / g_p;
+    // half the bending angle, beyond a right angle where the chord shortens again
+    double hp = asin(fmin(fabs(s), 1.0));
+    const double ct = fwd ? 1.0 : Cp * Lv + (pxf + g_tot * h) * xi;  // sign of cos(angle + phi_1 - theta)
+    if (ct < 0) hp = kPi - hp;
+    F = hp / fabs(s);
+    dF = (1 / cos(hp) - F) / (2 * q);
   }
-  double L_u = xi;
-  double L_v = -1 * (l * sinc_a + x * sin_a);
-  double L_c = sqrt(L_v * L_v + L_u * L_u);
-  double theta = atan2(L_u, -L_v);
-  double angle_p = 2 * (angle + phi_1 - theta);
-  double hp = angle_p / 2;
-  double S = 1, dS = 0;
-  if (fabs(hp) >= 1e-8) {
-    S = sin(hp) / hp;
-    dS = (hp * cos(hp) - sin(hp)) / (hp * hp);
+  const double Lp = Lc * F, w = Lp * ipt;
+  // directions: x, px, py, rel
+  const double d_ps[4] = {0, -px * ips, -py * ips, rel * ips};
+  const double d_pt2[4] = {0, 0, -py, rel};  // d(pt^2)/2
+  double jx[4], jp[4], jy[4], jz[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const double dh = i == 0 ? h0 * g : 0.0, dpx = i == 1 ? 1.0 : 0.0;
+    const double dpxf = ca * dpx + sa * d_ps[i] - g_tot * dh;
+    const double dR = (d_pt2[i] - pxf * dpxf) * iR;
+    const double dCp = ca * d_ps[i] - sa * dpx;
+    const double dxi = fwd ? (dh * N + h * (2 * dpxf + g_tot * dh) - xi * (dR + dCp)) * iD : (dR - dCp) * iD;
+    const double dLc = (xi * dxi + (i == 0 ? Lv * sa : 0.0)) * iLc;
+    const double dpt = d_pt2[i] * ipt * ipt;  // over pt
+    const double dLp = dLc * F + Lc * dF * (2 * q) * (dLc * iLc - dpt);
+    const double dw = dLp * ipt - w * dpt;
+    jx[i] = (i == 0 ? ca : 0.0) + dxi;
+    jp[i] = dpxf;
+    jy[i] = py * dw + (i == 2 ? w : 0.0);
+    jz[i] = -rel * dw - (i == 3 ? w : 0.0);
   }
-  double L_p = L_c / S;
-  double psi = phi_1 + angle - angle_p;
-  // reverse sweep
-  double b_pt = 0, b_rel = 0, b_Lp = 0, b_phi = 0, b_angp = 0, b_Lc = 0, b_Lu = 0, b_Lv = 0, b_xi = 0;
-  double b_alpha = 0, b_rad = 0, b_cp = 0, b_sp = 0, b_gp = 0, b_gx1 = 0, b_ls = 0;
-  double b_x = 0, b_px = 0, b_py = 0;
-  // z' = z + beta l / beta0 - rel L_p / pt
-  double beta_bar = a.beta + a.z * l / G.beta0;
-  b_rel += -a.z * L_p / pt;
-  b_Lp += -a.z * rel / pt;
-  b_pt += a.z * rel * L_p / (pt * pt);
-  // y' = y + py L_p / pt
-  b_py += a.y * L_p / pt;
-  b_Lp += a.y * py / pt;
-  b_pt += -a.y * py * L_p / (pt * pt);
-  // px' = pt sin(psi)
-  b_pt += a.px * sin(psi);
-  double b_psi = a.px * pt * cos(psi);
-  b_phi += b_psi;
-  b_angp += -b_psi;
-  // py' = py, pz' = pz
-  b_py += a.py;
-  double b_pz = a.pz;
-  // L_p = L_c / S(hp)
-  b_Lc += b_Lp / S;
-  double b_S = -b_Lp * L_c / (S * S);
-  b_angp += b_S * dS / 2;
-  // angle_p = 2 (angle + phi_1 - theta)
-  b_phi += 2 * b_angp;
-  double b_theta = -2 * b_angp;
-  double X = -L_v, Y = L_u, R2 = X * X + Y * Y;
-  b_Lu += b_theta * X / R2;
-  double b_X = -b_theta * Y / R2;
-  b_Lv += -b_X;
-  // L_c = sqrt(L_v^2 + L_u^2)
-  b_Lv += b_Lc * L_v / L_c;
-  b_Lu += b_Lc * L_u / L_c;
-  // L_v = -(l sinc_a + x sin_a), L_u = xi
-  b_x += -b_Lv * sin_a;
-  b_xi += b_Lu;
-  // x' = x cos_a - l^2 g cosc_a + xi
-  b_x += a.x * cos_a;
-  b_xi += a.x;
-  // xi
-  if (cp > 0) {
-    b_alpha += b_xi / den;
-    double b_den = -b_xi * alpha / (den * den);
-    b_rad += b_den;
-    b_cp += b_den;
-  } else {
-    b_rad += b_xi / g_p;
-    b_cp += -b_xi / g_p;
-    b_gp += -b_xi * (rad - cp) / (g_p * g_p);
+  const double zb = l / G.beta0;
+#pragma unroll
+  for (int i = 0; i < NC; i++) {
+    const Adj o = a[i];
+    a[i].x = o.x * jx[0] + o.px * jp[0] + o.y * jy[0] + o.z * jz[0];
+    a[i].px = o.x * jx[1] + o.px * jp[1] + o.y * jy[1] + o.z * jz[1];
+    a[i].py = o.py + o.x * jx[2] + o.px * jp[2] + o.y * jy[2] + o.z * jz[2];
+    a[i].pz = o.pz + o.x * jx[3] + o.px * jp[3] + o.y * jy[3] + o.z * jz[3];
+    a[i].beta = o.beta + o.z * zb;
   }
-  // rad = sqrt(r); r = cp^2 + g_p alpha
-  double b_r = b_rad / (2 * rad);
-  b_cp += b_r * 2 * cp;
-  b_gp += b_r * alpha;
-  b_alpha += b_r * g_p;
-  // alpha = 2 gx1 sp l sinc_a - g_p ls^2; ls = gx1 l sinc_a
-  b_gx1 += b_alpha * 2 * sp * l * sinc_a;
-  b_sp += b_alpha * 2 * gx1 * l * sinc_a;
-  b_gp += -b_alpha * ls * ls;
-  b_ls += -b_alpha * g_p * 2 * ls;
-  b_gx1 += b_ls * l * sinc_a;
-  b_x += b_gx1 * g;
-  // cp, sp of angle + phi_1
-  b_phi += -b_cp * sp + b_sp * cp;
-  // phi_1 = asin(px/pt)
-  double b_u = b_phi / sqrt(1 - u * u);
-  b_px += b_u / pt;
-  b_pt += -b_u * px / (pt * pt);
-  // g_p = g_tot / pt
-  b_pt += -b_gp * g_tot / (pt * pt);
-  // pt = sqrt(rel^2 - py^2)
-  b_rel += b_pt * rel / pt;
-  b_py += -b_pt * py / pt;
-  b_pz += b_rel;
-  a.x = b_x;
-  a.px = b_px;
-  a.py = b_py;
-  a.pz = b_pz;
-  a.beta = beta_bar;
-  // a.y and a.z pass through (y' = y + ..., z' = z + ...)
 }
 
 // apply_energy_kick: (pz, beta, z) with energy gain dE; g_dE receives dL/d(dE).
@@ -381,160 +369,192 @@ BG_HOST_DEVICE int adj_supported(const EleHdr& h) {
   }
 }
 
-// Reverse of one element body (the part between track1's checks) at input p (caches refreshed):
-// maps the cotangent of the element's output to that of its input; gscale += sum_c c dL/dc over
-// the element's strength coefficients.
-BG_HD void vjp_element(const EleHdr& h, const double* __restrict__ pool, const Particle& pin, Adj& a,
-                       double& gscale, const Globals& G) {
-  const double* b = pool + h.param;
+// Reverse of the RF cavity body (body_rf) for one cotangent.
+BG_COLD void vjp_rf(const EleHdr& h, const double* __restrict__ b, const Particle& pin, Adj& a1, double& gs1,
+                    const Globals& G) {
+  Adj a[1] = {a1};
+  double gscale[1] = {gs1};
   Particle p = pin;
-  switch (h.kind) {
-    case K_DRIFT:
-      vjp_drift(p, b[0], a, G);
-      return;
-    case K_QUAD: {
-      const int np = h.n_pole, n_step = h.n_step;
-      const double* kh = b + QD_FIXED;
-      const double* kf = kh + 2 * np;
-      const double* mis = kh + kick_doubles(np, n_step);
-      const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
-      const double b1 = b[0], length = b[1], sl = b[2];
-      AdjTape t;
-      if (misal) offset_set(p, mis, has_t);
-      for (int i = 0; i <= n_step; i++) {
-        if (i > 0) {
-          t.push(p);
-          quad_step(p, b1, length, sl, G);
-        }
-        if (np) {
-          t.push(p);
-          ab_kicks(p, (i == 0 || i == n_step) ? kh : kf, np);
-        }
-      }
-      if (misal && has_t) vjp_tilt(mis[2], -mis[3], a);
-      for (int i = n_step; i >= 0; i--) {
-        if (np) vjp_ab_kicks(t.in[--t.n], (i == 0 || i == n_step) ? kh : kf, np, a, gscale);
-        if (i > 0) vjp_quad_step(t.in[--t.n], b1, length, sl, a, gscale, G);
-      }
-      if (misal && has_t) vjp_tilt(mis[2], mis[3], a);
-      return;
-    }
-    case K_THICK: {
-      const int np = h.n_pole, n_step = h.n_step;
-      const double* kh = b + TH_FIXED;
-      const double* kf = kh + 2 * np;
-      const double* mis = kh + kick_doubles(np, n_step);
-      const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
-      const double sl = b[0];
-      AdjTape t;
-      if (misal) offset_set(p, mis, has_t);
-      for (int i = 0; i <= n_step; i++) {
-        if (i > 0) {
-          t.push(p);
-          drift(p, sl);
-        }
-        if (np) {
-          t.push(p);
-          ab_kicks(p, (i == 0 || i == n_step) ? kh : kf, np);
-        }
-      }
-      if (misal && has_t) vjp_tilt(mis[2], -mis[3], a);
-      for (int i = n_step; i >= 0; i--) {
-        if (np) vjp_ab_kicks(t.in[--t.n], (i == 0 || i == n_step) ? kh : kf, np, a, gscale);
-        if (i > 0) vjp_drift(t.in[--t.n], sl, a, G);
-      }
-      if (misal && has_t) vjp_tilt(mis[2], mis[3], a);
-      return;
-    }
-    case K_SBEND: {
-      const double* mis = b + SB_FIXED;
-      const bool misal = h.flags & F_MISALIGN;
-      AdjTape t;
-      if (misal) tilt(p, mis[2], mis[3]);
-      for (int n = 1; n <= h.n_step; n++) {
-        t.push(p);
-        if (h.flags & F_BEND_DRIFT) drift(p, b[0]);
-        else bend_exact_step(p, b, G);
-      }
-      if (misal) vjp_tilt(mis[2], -mis[3], a);
-      for (int n = h.n_step; n >= 1; n--) {
-        const Particle& q = t.in[--t.n];
-        if (h.flags & F_BEND_DRIFT) vjp_drift(q, b[0], a, G);
-        else vjp_bend_exact(q, b, a, G);
-      }
-      if (misal) vjp_tilt(mis[2], mis[3], a);
-      return;
-    }
-    case K_RFCAV: {
-      const int np = h.n_pole;
-      const double* kh = b + RF_FIXED;
-      const double* mis = kh + 2 * np;
-      const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
-      const double voltage = b[0], f = b[1], slice_len = b[4];
-      const int n_slice = h.n_step;
-      if (misal) offset_set(p, mis, has_t);
-      Particle pk0 = p;  // before the entrance kicks
-      if (np) ab_kicks(p, kh, np);
-      const Particle p_ph = p;  // the phase is taken here
-      double phase = rf_phase(p, b[2], f, b[3]);
-      // forward slices: K[i] = state before kick i, D[i] = state before drift i, phases
-      Particle Kin[kAdjMaxSteps + 1], Din[kAdjMaxSteps];
-      double ph[kAdjMaxSteps + 1];
-      for (int i = 0; i <= n_slice; i++) {
-        ph[i] = phase;
-        Kin[i] = p;
-        double dE = 1.0 * voltage * sin(phase) / n_slice;
-        if (i == 0 || i == n_slice) dE = dE / 2;
-        energy_kick(p, dE, G);
-        if (i != n_slice) {
-          refresh(p, G);
-          Din[i] = p;
-          double z = p.z;
-          drift(p, slice_len);
-          phase = phase + kTwoPi * f * (p.z - z) / (kCLight * p.beta);
-        }
-      }
+  const int np = h.n_pole;
+  const double* kh = b + RF_FIXED;
+  const double* mis = kh + 2 * np;
+  const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
+  const double voltage = b[0], f = b[1], slice_len = b[4];
+  const int n_slice = h.n_step;
+  if (misal) offset_set(p, mis, has_t);
+  Particle pk0 = p;  // before the entrance kicks
+  if (np) ab_kicks(p, kh, np);
+  const Particle p_ph = p;  // the phase is taken here
+  double phase = rf_phase(p, b[2], f, b[3]);
+  // forward slices: K[i] = state before kick i, D[i] = state before drift i, phases
+  Particle Kin[kAdjMaxSteps + 1], Din[kAdjMaxSteps];
+  double ph[kAdjMaxSteps + 1];
+  for (int i = 0; i <= n_slice; i++) {
+    ph[i] = phase;
+    Kin[i] = p;
+    double dE = 1.0 * voltage * sin(phase) / n_slice;
+    if (i == 0 || i == n_slice) dE = dE / 2;
+    energy_kick(p, dE, G);
+    if (i != n_slice) {
       refresh(p, G);
-      const Particle p_exit = p;  // before the exit kicks
-      if (misal && has_t) vjp_tilt(mis[2], -mis[3], a);
-      if (np) vjp_ab_kicks(p_exit, kh, np, a, gscale);
-      double b_phase = 0;
-      for (int i = n_slice; i >= 0; i--) {
-        if (i != n_slice) {
-          // phase_{i+1} = phase_i + 2 pi f (z_after - z_before) / (c beta), beta of Din[i]
-          const Particle& d = Din[i];
-          Particle e = d;
-          drift(e, slice_len);
-          double cfac = kTwoPi * f / (kCLight * d.beta);
-          a.z += b_phase * cfac;                // through z_after (the drift's output)
-          vjp_drift(d, slice_len, a, G);
-          a.z += -b_phase * cfac;               // z_before
-          a.beta += -b_phase * cfac * (e.z - d.z) / d.beta;
-        }
-        double dE = 1.0 * voltage * sin(ph[i]) / n_slice;
-        double dEfac = 1.0 * voltage / n_slice;
-        if (i == 0 || i == n_slice) {
-          dE = dE / 2;
-          dEfac = dEfac / 2;
-        }
-        double g_dE = 0;
-        vjp_energy_kick(Kin[i], dE, a, g_dE, G);
-        b_phase += g_dE * dEfac * cos(ph[i]);
-      }
-      // phase0 = modulo2(2 pi (phi0 - t f) + ..., pi), t = -z / (beta c)
-      double dt_dz = -1 / (p_ph.beta * kCLight), dt_dbeta = p_ph.z / (p_ph.beta * p_ph.beta * kCLight);
-      a.z += b_phase * (-kTwoPi * f) * dt_dz;
-      a.beta += b_phase * (-kTwoPi * f) * dt_dbeta;
-      if (np) vjp_ab_kicks(pk0, kh, np, a, gscale);
-      if (misal && has_t) vjp_tilt(mis[2], mis[3], a);
-      return;
+      Din[i] = p;
+      double z = p.z;
+      drift(p, slice_len);
+      phase = phase + kTwoPi * f * (p.z - z) / (kCLight * p.beta);
     }
-    default:
-      return;  // marker
+  }
+  refresh(p, G);
+  const Particle p_exit = p;  // before the exit kicks
+  if (misal && has_t) vjp_tilt<1>(mis[2], -mis[3], a);
+  if (np) vjp_ab_kicks<1>(p_exit, kh, np, a, gscale);
+  double b_phase = 0;
+  for (int i = n_slice; i >= 0; i--) {
+    if (i != n_slice) {
+      // phase_{i+1} = phase_i + 2 pi f (z_after - z_before) / (c beta), beta of Din[i]
+      const Particle& d = Din[i];
+      Particle e = d;
+      drift(e, slice_len);
+      double cfac = kTwoPi * f / (kCLight * d.beta);
+      a[0].z += b_phase * cfac;                // through z_after (the drift's output)
+      vjp_drift<1>(d, adj_caches(d, G), slice_len, a);
+      a[0].z += -b_phase * cfac;               // z_before
+      a[0].beta += -b_phase * cfac * (e.z - d.z) / d.beta;
+    }
+    double dE = 1.0 * voltage * sin(ph[i]) / n_slice;
+    double dEfac = 1.0 * voltage / n_slice;
+    if (i == 0 || i == n_slice) {
+      dE = dE / 2;
+      dEfac = dEfac / 2;
+    }
+    double g_dE = 0;
+    vjp_energy_kick(Kin[i], dE, a[0], g_dE, G);
+    b_phase += g_dE * dEfac * cos(ph[i]);
+  }
+  // phase0 = modulo2(2 pi (phi0 - t f) + ..., pi), t = -z / (beta c)
+  double dt_dz = -1 / (p_ph.beta * kCLight), dt_dbeta = p_ph.z / (p_ph.beta * p_ph.beta * kCLight);
+  a[0].z += b_phase * (-kTwoPi * f) * dt_dz;
+  a[0].beta += b_phase * (-kTwoPi * f) * dt_dbeta;
+  if (np) vjp_ab_kicks<1>(pk0, kh, np, a, gscale);
+  if (misal && has_t) vjp_tilt<1>(mis[2], mis[3], a);
+  a1 = a[0];
+  gs1 = gscale[0];
+}
+
+// Reverse of a body of several steps (quadrupole, thick multipole, bend), its sub-step inputs on a tape.
+template <int NC>
+BG_COLD void vjp_steps(const EleHdr& h, const double* __restrict__ b, const Particle& pin, const AdjCache& k,
+                       Adj* __restrict__ ap, double* __restrict__ gp, const Globals& G) {
+  Adj a[NC];
+  double gscale[NC];
+  for (int c = 0; c < NC; c++) {
+    a[c] = ap[c];
+    gscale[c] = gp[c];
+  }
+  Particle p = pin;
+  const int np = h.n_pole, n_step = h.n_step;
+  const bool quad = h.kind == K_QUAD, bend = h.kind == K_SBEND;
+  const double* kh = b + (quad ? QD_FIXED : TH_FIXED);
+  const double* kf = kh + 2 * np;
+  const double* mis = bend ? b + SB_FIXED : kh + kick_doubles(np, n_step);
+  const bool has_t = h.flags & F_TILT, misal = h.flags & F_MISALIGN;
+  AdjTape t;
+  if (misal) {
+    if (bend) tilt(p, mis[2], mis[3]);
+    else offset_set(p, mis, has_t);
+  }
+  for (int i = bend ? 1 : 0; i <= n_step; i++) {
+    if (i > 0) {
+      t.push(p);
+      if (quad) quad_step(p, b[0], b[1], b[2], G);
+      else if (bend && !(h.flags & F_BEND_DRIFT)) bend_exact_step(p, b, G);
+      else drift(p, b[0]);
+    }
+    if (np) {
+      t.push(p);
+      ab_kicks(p, (i == 0 || i == n_step) ? kh : kf, np);
+    }
+  }
+  if (misal && (bend || has_t)) vjp_tilt<NC>(mis[2], -mis[3], a);
+  for (int i = n_step; i >= (bend ? 1 : 0); i--) {
+    if (np) vjp_ab_kicks<NC>(t.in[--t.n], (i == 0 || i == n_step) ? kh : kf, np, a, gscale);
+    if (i > 0) {
+      const Particle& q = t.in[--t.n];
+      if (quad) vjp_quad_step<NC>(q, k, b[0], b[1], b[2], a, gscale);
+      else if (bend && !(h.flags & F_BEND_DRIFT)) vjp_bend_exact<NC>(q, k, b, a, G);
+      else vjp_drift<NC>(q, k, b[0], a);
+    }
+  }
+  if (misal && (bend || has_t)) vjp_tilt<NC>(mis[2], mis[3], a);
+  for (int c = 0; c < NC; c++) {
+    ap[c] = a[c];
+    gp[c] = gscale[c];
   }
 }
 
-// ---- per-particle driver: forward with checkpoints, then the reverse sweep -------------------
+// Reverse of one element body (the part between track1's checks) at input p (caches refreshed, k its
+// adj_caches): maps the cotangents of the element's output to those of its input; gscale += sum_c c dL/dc
+// over the element's strength coefficients.
+template <int NC>
+BG_HD void vjp_element(const EleHdr& h, const double* __restrict__ pool, const Particle& pin, const AdjCache& k,
+                       Adj (&a)[NC], double (&gscale)[NC], const Globals& G) {
+  const double* b = pool + h.param;
+  const bool misal = h.flags & F_MISALIGN, has_t = h.flags & F_TILT;
+  const int np = h.n_pole;
+  if (h.kind == K_DRIFT) {
+    vjp_drift<NC>(pin, k, b[0], a);
+  } else if (h.kind == K_QUAD && np == 0 && h.n_step == 1) {
+    const double* mis = b + QD_FIXED;
+    Particle p = pin;
+    if (misal) offset_set(p, mis, has_t);
+    if (misal && has_t) vjp_tilt<NC>(mis[2], -mis[3], a);
+    vjp_quad_step<NC>(p, k, b[0], b[1], b[2], a, gscale);
+    if (misal && has_t) vjp_tilt<NC>(mis[2], mis[3], a);
+  } else if (h.kind == K_THICK && np > 0 && h.n_step == 1) {
+    const double* kh = b + TH_FIXED;
+    const double* mis = kh + kick_doubles(np, 1);
+    Particle p0 = pin;
+    if (misal) offset_set(p0, mis, has_t);
+    Particle p1 = p0;
+    ab_kicks(p1, kh, np, h.flags & F_KICK_B_FROM2);
+    Particle p2 = p1;
+    drift(p2, b[0]);
+    if (misal && has_t) vjp_tilt<NC>(mis[2], -mis[3], a);
+    vjp_ab_kicks<NC>(p2, kh, np, a, gscale);
+    vjp_drift<NC>(p1, k, b[0], a);
+    vjp_ab_kicks<NC>(p0, kh, np, a, gscale);
+    if (misal && has_t) vjp_tilt<NC>(mis[2], mis[3], a);
+  } else if (h.kind == K_SBEND && h.n_step == 1 && !misal && !(h.flags & F_BEND_DRIFT)) {
+    vjp_bend_exact<NC>(pin, k, b, a, G);
+  } else if (h.kind == K_RFCAV) {
+    for (int c = 0; c < NC; c++) vjp_rf(h, b, pin, a[c], gscale[c], G);
+  } else if (h.kind != K_MARKER) {
+    Adj t[NC];
+    double g[NC];
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      t[c] = a[c];
+      g[c] = gscale[c];
+    }
+    vjp_steps<NC>(h, b, pin, k, t, g, G);
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      a[c] = t[c];
+      gscale[c] = g[c];
+    }
+  }
+}
+BG_HD void vjp_element(const EleHdr& h, const double* __restrict__ pool, const Particle& pin, Adj& a, double& gscale,
+                       const Globals& G) {
+  Adj t[1] = {a};
+  double g[1] = {gscale};
+  vjp_element<1>(h, pool, pin, adj_caches(pin, G), t, g, G);
+  a = t[0];
+  gscale = g[0];
+}
+
+// ---- per-particle driver of the host check: forward with checkpoints, then the reverse sweep ----
+// (the device spreads the same sweep over turns and particles, adjoint.cu)
+#if !defined(__CUDACC__)
 //
 // Loss: sum over particles alive after n_turns of loss_scale * (x^2 + y^2). Buffers are
 // structure-of-arrays with particle stride N: row r, component k of particle j at
@@ -651,5 +671,7 @@ BG_HD void adj_particle(const AdjArgs& a, int64_t j) {
     }
   }
 }
+
+#endif  // !__CUDACC__
 
 }  // namespace bmadgpu
