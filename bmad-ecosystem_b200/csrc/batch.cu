@@ -96,9 +96,9 @@ struct Variant {
   {B, M, (const void*)k_batch_track<B, M, false, true>, (const void*)k_batch_track<B, M, false, false>}
 #endif
 const Variant kVariants[] = {
-    BG_BATCH_VARIANT(64, 8),  BG_BATCH_VARIANT(64, 12), BG_BATCH_VARIANT(128, 3), BG_BATCH_VARIANT(128, 4),
-    BG_BATCH_VARIANT(128, 5), BG_BATCH_VARIANT(128, 6), BG_BATCH_VARIANT(256, 1), BG_BATCH_VARIANT(256, 2),
-    BG_BATCH_VARIANT(256, 3), BG_BATCH_VARIANT(512, 1),
+    BG_BATCH_VARIANT(64, 4),  BG_BATCH_VARIANT(64, 8),  BG_BATCH_VARIANT(64, 12), BG_BATCH_VARIANT(128, 3),
+    BG_BATCH_VARIANT(128, 4), BG_BATCH_VARIANT(128, 5), BG_BATCH_VARIANT(128, 6), BG_BATCH_VARIANT(256, 1),
+    BG_BATCH_VARIANT(256, 2), BG_BATCH_VARIANT(256, 3), BG_BATCH_VARIANT(512, 1),
 };
 #undef BG_BATCH_VARIANT
 
@@ -115,6 +115,9 @@ cudaError_t batch_upload_constants() {
 }
 
 cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_count, BatchKernel* out) {
+#if defined(BG_FAST_MAPS)
+  smem_bytes = 0;  // this build's kernels do not stage (batch_kernel.cuh)
+#endif
   // same register-budget selection as launch_track
   const Variant* v = nullptr;
   for (const Variant& k : kVariants) {

@@ -20,7 +20,7 @@ const void* batch_rec_kernel(int block, int minb, bool full) {
 #define BG_BATCH_REC(B, M) {B, M, (const void*)k_batch_track<B, M, true, true>, (const void*)k_batch_track<B, M, true, false>}
 #endif
   static const Entry kRec[] = {
-      BG_BATCH_REC(64, 8),  BG_BATCH_REC(64, 12), BG_BATCH_REC(128, 3), BG_BATCH_REC(128, 4),
+      BG_BATCH_REC(64, 4),  BG_BATCH_REC(64, 8),  BG_BATCH_REC(64, 12), BG_BATCH_REC(128, 3), BG_BATCH_REC(128, 4),
       BG_BATCH_REC(128, 5), BG_BATCH_REC(128, 6), BG_BATCH_REC(256, 1), BG_BATCH_REC(256, 2),
       BG_BATCH_REC(256, 3), BG_BATCH_REC(512, 1),
   };

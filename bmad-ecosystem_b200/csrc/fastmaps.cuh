@@ -120,7 +120,8 @@ BG_HD Pair load2(const double* __restrict__ b) {
 #endif
 }
 
-// The coordinates that change inside an element (pz and beta do not in these maps).
+// The coordinates that change inside an element (pz and beta do not in these maps): a copy to work on
+// where a range is tested after some of them have changed. The maps take it or the particle itself.
 struct Orbit {
   double x, px, y, py, z;
 };
@@ -129,7 +130,8 @@ struct Orbit {
 
 // track_a_drift: with P = px/rel, Q = py/rel, e = P^2 + Q^2, px/ps = P (1 + v) and
 // dz = L (beta/beta0 - 1 - v), v = rel/ps - 1. Range: e < 2^-12.
-BG_HD bool drift_f(Orbit& o, const Particle& c, double L) {
+template <class T>
+BG_HD bool drift_f(T& o, const Particle& c, double L) {
   const double P = o.px * c.e_factor, Q = o.py * c.e_factor;
   const double e = fma(P, P, Q * Q);
   if ((uint32_t)hi_word(e) >= kHi2m12) return false;  // NaN too
@@ -145,7 +147,8 @@ BG_HD bool drift_f(Orbit& o, const Particle& c, double L) {
 // With u = k step^2: cos(sqrt u) = E - u O, cosh = E + u O, E and O series in u^2; likewise
 // sin(sqrt u)/sqrt u and sinh(sqrt u)/sqrt u. Truncation below 2^-55 for |u| < 1/2. k < 0 (u < 0)
 // exchanges the planes in the same formulas.
-BG_HD bool quad_step_f(Orbit& o, const Particle& q, const double* __restrict__ b) {
+template <class T>
+BG_HD bool quad_step_f(T& o, const Particle& q, const double* __restrict__ b) {
   const double ef = q.e_factor;
   const double u = b[4] * ef;
   if (hi_abs(u) >= kHiHalf) return false;
@@ -229,7 +232,8 @@ BG_HD bool kicks_f(Orbit& o, const double* __restrict__ c, int np, bool b_from2)
   return true;
 }
 // The same for a sextupole alone: S = b_2 (x + i y)^2.
-BG_HD void kick2_f(Orbit& o, double b2) {
+template <class T>
+BG_HD void kick2_f(T& o, double b2) {
   o.px = fma(-b2, fma(o.x, o.x, -(o.y * o.y)), o.px);
   o.py = fma(2 * b2, o.x * o.y, o.py);
 }
@@ -280,7 +284,8 @@ BG_HD bool frame_f(Orbit& o, const Particle& q, const double* __restrict__ m) {
 
 // hwang_bend_edge_kick for upright faces without a fringe integral or field index: only the gs2
 // terms are left, gs2 = g_tot.
-BG_HD void upright_edge_f(Orbit& o, double ef, double g) {
+template <class T>
+BG_HD void upright_edge_f(T& o, double ef, double g) {
   const double h = 0.5 * g * ef, yy = o.y * o.y, q = h * o.px;
   o.z = fma(-(q * ef), yy, o.z);
   o.py = fma(-2 * q, o.y, o.py);
@@ -288,7 +293,8 @@ BG_HD void upright_edge_f(Orbit& o, double ef, double g) {
 }
 
 // hwang_bend_edge_kick in full; e: the edge's coefficients (table.h).
-BG_HD void hwang_edge_f(Orbit& o, double ef, const double* __restrict__ e, bool entering) {
+template <class T>
+BG_HD void hwang_edge_f(T& o, double ef, const double* __restrict__ e, bool entering) {
   const double gt = e[0], gt2 = e[1], gs2 = e[2], k1t = e[3], fg = e[4], gtot = e[5], cdpx = e[6];
   const double sg = entering ? 1.0 : -1.0;
   const double v1 = o.x, v2 = o.px, v3 = o.y, v4 = o.py;
@@ -325,7 +331,8 @@ BG_HD void hwang_edge_f(Orbit& o, double ef, const double* __restrict__ e, bool 
 // Range: the momentum series' e < 2^-12 at both ends; L_c^2/L_c0^2 - 1 and q - q0 below 2^-8, where
 // their series, truncated at the sixth power, are good to 2^-58; clear of the reference's semi-linear
 // map near the zero orbit (track_a_bend.f90:136-159, all of |px|, |py|, |pz| < 1e-9).
-BG_HD bool bend_step_f(Orbit& o, const Particle& q, const double* __restrict__ b, const Globals& G, bool has_dg) {
+template <class T>
+BG_HD bool bend_step_f(T& o, const Particle& q, const double* __restrict__ b, const Globals& G, bool has_dg) {
   const Pair gl = load2(b + SB_F), cs = load2(b + SB_F + 2), ht = load2(b + SB_F + 4), xh = load2(b + SB_F + 6);
   const double g = gl.a, L = gl.b, ca = cs.a, sa = cs.b, h0 = ht.a;
   const double x = o.x, px = o.px, py = o.py, pz = q.pz, ef = q.e_factor;
@@ -389,6 +396,21 @@ BG_HD bool element_f(Particle& p, const EleHdr* __restrict__ h, const FastHdr& f
   const uint32_t c = f.code;
   const bool mis = c & FC_MISALIGN, tilted = c & FC_TILT;
   if ((c & FC_ENTRANCE) && !((hi_abs(p.x) < f.acc_x) & (hi_abs(p.y) < f.acc_y))) return false;
+  if (!(c & (FC_MISALIGN | FC_PITCH))) {  // nothing moves before the range is tested: in place
+    switch (c & FC_BODY) {
+      case FC_DRIFT: return drift_f(p, p, b[0]);
+      case FC_QUAD: return quad_step_f(p, p, b);
+      case FC_BEND:
+        if (c & FC_EDGE_IN) break;
+        if (!bend_step_f(p, p, b, G, c & FC_DG)) return false;
+        if (c & FC_EDGE_OUT) {
+          if (c & FC_UPRIGHT) upright_edge_f(p, p.e_factor, -b[2]);
+          else hwang_edge_f(p, p.e_factor, b + SB_EDGE_OUT, false);
+        }
+        return true;
+      default: break;
+    }
+  }
   Orbit o = {p.x, p.px, p.y, p.py, p.z};
   // misalign of a pitched quadrupole or thick multipole
   const int m = tilted && (c & FC_PITCH)

@@ -574,12 +574,19 @@ std::vector<double> bend_frame_block(const bmadgpu_element& e) {
   return blk;
 }
 
+// A bend's entries from SB_F and what they were made from (push_bend_series).
+struct BendSeries {
+  double step_len = 0, g = 0, g_tot = 0;
+  std::vector<double> v;
+};
+
 struct Packer {
   std::vector<EleHdr> hdr;
   std::vector<ApRec> ap;
   std::vector<double> pool;
   std::map<std::vector<double>, uint32_t> dedupe;
   std::map<std::vector<double>, uint16_t> ap_dedupe;
+  BendSeries bend;
 
   uint32_t add_block(const std::vector<double>& blk) {
     if (blk.empty()) return 0;
@@ -733,8 +740,14 @@ FastHdr fast_header(const EleHdr& h, uint16_t flags, const std::vector<double>& 
   return f;
 }
 
-// The K_SBEND entries from SB_F (table.h), from extended-precision values rounded once.
-void push_bend_series(std::vector<double>& blk, double step_len, double g, double g_tot) {
+// The K_SBEND entries from SB_F (table.h), from extended-precision values rounded once. last: the
+// previous bend's inputs and entries, since a ring's bends are mostly alike.
+void push_bend_series(std::vector<double>& blk, double step_len, double g, double g_tot, BendSeries& last) {
+  if (!last.v.empty() && last.step_len == step_len && last.g == g && last.g_tot == g_tot) {
+    blk.insert(blk.end(), last.v.begin(), last.v.end());
+    return;
+  }
+  const size_t at = blk.size();
   typedef long double X;
   const X L = step_len, a = (X)g * L, h = a / 2, s = std::sin(h), c = std::cos(h);
   const X sinc = a == 0 ? 1 : 2 * s * c / a, cosc = a == 0 ? (X)0.5 : 2 * s * s / (a * a);
@@ -761,6 +774,10 @@ void push_bend_series(std::vector<double>& blk, double step_len, double g, doubl
                          (double)Lc2, (double)((X)g_tot * (X)g_tot / 4), (double)Lc});
   for (X v : f) blk.push_back((double)v);
   blk.push_back(g_tot == g ? 0.0 : (double)(Lc * f[0] - L));
+  last.step_len = step_len;
+  last.g = g;
+  last.g_tot = g_tot;
+  last.v.assign(blk.begin() + at, blk.end());
 }
 
 void push_kicks(std::vector<double>& blk, const double* a, const double* b, int n_pole, double scale) {
@@ -1088,7 +1105,7 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
             double cdpx = gt * ge * (1 + 2 * (tan_e * tan_e));
             blk.insert(blk.end(), {gt, gt2, gs2, k1_tane, fg_factor, ge, cdpx});
           }
-          push_bend_series(blk, step_len, g, g_tot);
+          push_bend_series(blk, step_len, g, g_tot, pk.bend);
           if (e.fringe_type == BMADGPU_FRINGE_BASIC_BEND || e.fringe_type == BMADGPU_FRINGE_HARD_EDGE_ONLY) {
             if (e.fringe_at == BMADGPU_ENTRANCE_END || e.fringe_at == BMADGPU_BOTH_ENDS) flags |= F_EDGE_IN;
             if (e.fringe_at == BMADGPU_EXIT_END || e.fringe_at == BMADGPU_BOTH_ENDS) flags |= F_EDGE_OUT;

@@ -73,7 +73,7 @@ __device__ __forceinline__ bool track_turn(Particle& p, const EleHdr* __restrict
                                            const ApRec* __restrict__ ap, const Globals& G, int ix_start, int ix_end,
                                            bool first_turn, int turn_no, LossInfo& li) {
 #if defined(BG_FAST_MAPS)
-  if (!REF) {
+  if constexpr (!REF) {
     if (first_turn) p.hot = p.hot && entry_f(p, G);
     FastHdr next;  // the next element's, loaded while this one's arithmetic runs
     load_fast(hdr, ix_start, next);
@@ -89,20 +89,22 @@ __device__ __forceinline__ bool track_turn(Particle& p, const EleHdr* __restrict
       }
     }
     return true;
-  }
+  } else
 #endif
-  for (int ie = ix_start; ie < ix_end; ++ie) {
-    EleHdr h;
-    load_hdr(hdr, ie, h);
-    int loc = track1<FULL>(p, h, pool, ap, G, first_turn && ie == ix_start);
-    if (loc) {
-      li.loc = loc;
-      li.ele = ie;
-      li.turn = turn_no;
-      return false;
+  {
+    for (int ie = ix_start; ie < ix_end; ++ie) {
+      EleHdr h;
+      load_hdr(hdr, ie, h);
+      int loc = track1<FULL>(p, h, pool, ap, G, first_turn && ie == ix_start);
+      if (loc) {
+        li.loc = loc;
+        li.ele = ie;
+        li.turn = turn_no;
+        return false;
+      }
     }
+    return true;
   }
-  return true;
 }
 
 // Writes a particle back after a launch of n_turns turns starting at turn turn0. Particles that
