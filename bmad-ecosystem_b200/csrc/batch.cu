@@ -3,8 +3,9 @@
 // k_batch_track: a persistent grid (one full wave of CTAs) pulls work items from a device
 // counter. An item is (variant, tile of `tile` consecutive entries of the variant's live list);
 // items of variant v are numbered tile_prefix[v] .. tile_prefix[v+1]-1. A CTA that moves to a
-// new variant re-stages that variant's element table into shared memory with a bulk copy
-// (mbarrier completion, bounded wait, the phase bit flipping on every use). Each thread tracks
+// new variant takes up that variant's element table: the default build reads it from global memory
+// through L1, the correctly rounded one re-stages it into shared memory with a bulk copy (mbarrier
+// completion, bounded wait, the phase bit flipping on every use). Each thread tracks
 // `ppt` particles of the tile one after another, each through all turns of the launch, with the
 // same per-particle code as k_track (particle.cuh). Survivors are appended to the variant's next
 // live list with a warp ballot and one atomic per warp, so compaction needs no extra pass.

@@ -7,12 +7,10 @@
 // that the reference recomputes from element attributes alone come precomputed from the packed
 // table with the same expressions, hence bit-identical. Functions of pz alone that the reference
 // recomputes per element with the same expression are cached in the particle (refresh()).
-// The kernels are compiled without FMA contraction, so the device results differ from the
-// reference's only through the six transcendentals the maps call (sin, cos, asin, atan2, sinh,
-// cosh). The library is built twice from this source: with the device libm (libbmadgpu.so, the
-// fast build), and with BG_CR_MATH, where those six are correctly rounded (crmath.cuh) and the
-// results are bit for bit those of the reference's algorithm run with a correctly rounded libm
-// (libbmadgpu_cr.so).
+// The kernels are compiled without FMA contraction. With BG_CR_MATH (libbmadgpu_cr.so) the
+// transcendentals the maps call are correctly rounded (crmath.cuh) and the results are bit for bit those
+// of the reference's algorithm run with a correctly rounded libm. The default build (libbmadgpu.so)
+// tracks with the forms of fastmaps.cuh and comes here, with the device libm, for what they do not cover.
 #pragma once
 #include <math.h>
 #include <stdint.h>

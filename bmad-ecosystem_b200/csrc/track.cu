@@ -4,8 +4,8 @@
 // the launch, running the element loop of track_bunch (bmad/multiparticle/beam_mod.f90:159-166)
 // with the per-element wrapper of track1 (bmad/code/track1.f90:179-329) around each map. The
 // packed element table is staged once per CTA into shared memory by a TMA bulk copy
-// (cp.async.bulk, mbarrier completion, bounded wait), so the element loop reads invariants with
-// broadcast shared-memory loads. Lost particles leave the loop at once and record where they
+// (cp.async.bulk, mbarrier completion, bounded wait) where that costs no residency, and read through L1
+// otherwise. Lost particles leave the loop at once and record where they
 // were lost (state, element, turn, location) as track1_bunch_hom leaves them
 // (bmad/multiparticle/beam_utils.f90:81-86). Optional per-turn sums over live particles
 // (n_live, <x_i>, <x_i x_j>; bsim/modules/lt_tracking_mod.f90:2393-2421) are reduced with warp
