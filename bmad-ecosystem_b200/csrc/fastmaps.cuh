@@ -328,7 +328,8 @@ BG_HD void hwang_edge_f(T& o, double ef, const double* __restrict__ e, bool ente
 // design length, about 1e-4 of it, is not formed by subtracting the two.
 // beta L / beta0 is rounded as the reference rounds it: that rounding is the same in every bend of a
 // turn, so it is the one term whose last bit shows in z against the reference's tracking.
-// Range: the momentum series' e < 2^-12 at both ends; L_c^2/L_c0^2 - 1 and q - q0 below 2^-8, where
+// Range: a step length above zero (fast_header), the chord and the arc being positive;
+// the momentum series' e < 2^-12 at both ends; L_c^2/L_c0^2 - 1 and q - q0 below 2^-8, where
 // their series, truncated at the sixth power, are good to 2^-58; clear of the reference's semi-linear
 // map near the zero orbit (track_a_bend.f90:136-159, all of |px|, |py|, |pz| < 1e-9).
 template <class T>

@@ -715,7 +715,9 @@ FastHdr fast_header(const EleHdr& h, uint16_t flags, const std::vector<double>& 
         if (!(flags & (F_EDGE_IN | F_EDGE_OUT | F_MISALIGN))) c = FC_DRIFT;
         break;
       }
-      if (!(std::fabs(blk[1] * blk[0]) < 1) || !(std::fabs(blk[2] * blk[0]) < 1)) break;
+      // bend_step_f's arc deviates from the design arc, which a negative length (whose arc the reference
+      // takes the long way round) does not have
+      if (!(blk[0] > 0) || !(std::fabs(blk[1] * blk[0]) < 1) || !(std::fabs(blk[2] * blk[0]) < 1)) break;
       bool upright = true;  // gt, gt2, k1_tane, fg_factor and the entrance dpx coefficient zero, gs2 = g_tot
       for (int end = 0; end < 2; end++) {
         const double* e = &blk[end == 0 ? SB_EDGE_IN : SB_EDGE_OUT];
