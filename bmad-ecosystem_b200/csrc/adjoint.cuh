@@ -207,12 +207,137 @@ BG_HD void vjp_tilt(double c, double s, Adj (&a)[NC]) {
   }
 }
 
+// Exact sbend body step in the trigonometric variables of bend_exact_step itself, one cotangent: for the
+// bends that vjp_bend_exact's range leaves out (negative lengths, whose arc goes the long way round, and
+// angles beyond a quarter turn, whose half angle asin does not give).
+BG_COLD void vjp_bend_trig(const Particle& p, const double* __restrict__ b, Adj& a, const Globals& G) {
+  double l = b[0], g = b[1], g_tot = b[2], angle = b[4];
+  double cos_a = b[5], sin_a = b[6], sinc_a = b[7];
+  double x = p.x, px = p.px, py = p.py, pz = p.pz;
+  double rel = 1 + pz;
+  // forward intermediates
+  double pt = sqrt(rel * rel - py * py);
+  double g_p = g_tot / pt;
+  double u = px / pt;
+  double phi_1 = asin(u);
+  double cp = cos(angle + phi_1), sp = sin(angle + phi_1);
+  double gx1 = 1 + g * x;
+  double ls = gx1 * l * sinc_a;
+  double alpha = 2 * gx1 * sp * l * sinc_a - g_p * (ls * ls);
+  double r = cp * cp + g_p * alpha;
+  double rad = sqrt(r);
+  double xi, den = 0;
+  if (cp > 0) {
+    den = rad + cp;
+    xi = alpha / den;
+  } else {
+    xi = (rad - cp) / g_p;
+  }
+  double L_u = xi;
+  double L_v = -1 * (l * sinc_a + x * sin_a);
+  double L_c = sqrt(L_v * L_v + L_u * L_u);
+  double theta = atan2(L_u, -L_v);
+  double angle_p = 2 * (angle + phi_1 - theta);
+  double hp = angle_p / 2;
+  double S = 1, dS = 0;
+  if (fabs(hp) >= 1e-8) {
+    S = sin(hp) / hp;
+    dS = (hp * cos(hp) - sin(hp)) / (hp * hp);
+  }
+  double L_p = L_c / S;
+  double psi = phi_1 + angle - angle_p;
+  // reverse sweep
+  double b_pt = 0, b_rel = 0, b_Lp = 0, b_phi = 0, b_angp = 0, b_Lc = 0, b_Lu = 0, b_Lv = 0, b_xi = 0;
+  double b_alpha = 0, b_rad = 0, b_cp = 0, b_sp = 0, b_gp = 0, b_gx1 = 0, b_ls = 0;
+  double b_x = 0, b_px = 0, b_py = 0;
+  // z' = z + beta l / beta0 - rel L_p / pt
+  double beta_bar = a.beta + a.z * l / G.beta0;
+  b_rel += -a.z * L_p / pt;
+  b_Lp += -a.z * rel / pt;
+  b_pt += a.z * rel * L_p / (pt * pt);
+  // y' = y + py L_p / pt
+  b_py += a.y * L_p / pt;
+  b_Lp += a.y * py / pt;
+  b_pt += -a.y * py * L_p / (pt * pt);
+  // px' = pt sin(psi)
+  b_pt += a.px * sin(psi);
+  double b_psi = a.px * pt * cos(psi);
+  b_phi += b_psi;
+  b_angp += -b_psi;
+  // py' = py, pz' = pz
+  b_py += a.py;
+  double b_pz = a.pz;
+  // L_p = L_c / S(hp)
+  b_Lc += b_Lp / S;
+  double b_S = -b_Lp * L_c / (S * S);
+  b_angp += b_S * dS / 2;
+  // angle_p = 2 (angle + phi_1 - theta)
+  b_phi += 2 * b_angp;
+  double b_theta = -2 * b_angp;
+  double X = -L_v, Y = L_u, R2 = X * X + Y * Y;
+  b_Lu += b_theta * X / R2;
+  double b_X = -b_theta * Y / R2;
+  b_Lv += -b_X;
+  // L_c = sqrt(L_v^2 + L_u^2)
+  b_Lv += b_Lc * L_v / L_c;
+  b_Lu += b_Lc * L_u / L_c;
+  // L_v = -(l sinc_a + x sin_a), L_u = xi
+  b_x += -b_Lv * sin_a;
+  b_xi += b_Lu;
+  // x' = x cos_a - l^2 g cosc_a + xi
+  b_x += a.x * cos_a;
+  b_xi += a.x;
+  // xi
+  if (cp > 0) {
+    b_alpha += b_xi / den;
+    double b_den = -b_xi * alpha / (den * den);
+    b_rad += b_den;
+    b_cp += b_den;
+  } else {
+    b_rad += b_xi / g_p;
+    b_cp += -b_xi / g_p;
+    b_gp += -b_xi * (rad - cp) / (g_p * g_p);
+  }
+  // rad = sqrt(r); r = cp^2 + g_p alpha
+  double b_r = b_rad / (2 * rad);
+  b_cp += b_r * 2 * cp;
+  b_gp += b_r * alpha;
+  b_alpha += b_r * g_p;
+  // alpha = 2 gx1 sp l sinc_a - g_p ls^2; ls = gx1 l sinc_a
+  b_gx1 += b_alpha * 2 * sp * l * sinc_a;
+  b_sp += b_alpha * 2 * gx1 * l * sinc_a;
+  b_gp += -b_alpha * ls * ls;
+  b_ls += -b_alpha * g_p * 2 * ls;
+  b_gx1 += b_ls * l * sinc_a;
+  b_x += b_gx1 * g;
+  // cp, sp of angle + phi_1
+  b_phi += -b_cp * sp + b_sp * cp;
+  // phi_1 = asin(px/pt)
+  double b_u = b_phi / sqrt(1 - u * u);
+  b_px += b_u / pt;
+  b_pt += -b_u * px / (pt * pt);
+  // g_p = g_tot / pt
+  b_pt += -b_gp * g_tot / (pt * pt);
+  // pt = sqrt(rel^2 - py^2)
+  b_rel += b_pt * rel / pt;
+  b_py += -b_pt * py / pt;
+  b_pz += b_rel;
+  a.x = b_x;
+  a.px = b_px;
+  a.py = b_py;
+  a.pz = b_pz;
+  a.beta = beta_bar;
+  // a.y and a.z pass through (y' = y + ..., z' = z + ...)
+}
+
 // Exact sbend body step (bend_exact_step). In the momentum components of the rotated axes (Sp, Cp) and
 // the exit components (pxf, R) the map has no trigonometric function of the particle but the arc over
 // its chord, L_p = L_c F(q), F = asin(s)/s, q = s^2 = (g_tot L_c / 2 pt)^2:
 //   pxf = ca px + sa ps - g_tot h, h = (1 + g x) L sinc, xi = h (2 pxf + g_tot h) / (R + Cp),
 //   x' = x ca + xi - const, y' = y + py L_p / pt, z' = z + beta L / beta0 - rel L_p / pt.
-// Four directions (x, px, py, rel) are differentiated through it.
+// Four directions (x, px, py, rel) are differentiated through it. Range: the half bending angle below a
+// right angle, so that F is asin's: a positive length, an angle up to 1.5 (below a quarter turn), and the
+// cosine of the half angle, (Cp L_v + Sp xi) / (pt L_c), above zero; Cp > 0 for the quotient by R + Cp.
 template <int NC>
 BG_HD void vjp_bend_exact(const Particle& p, const AdjCache& k, const double* __restrict__ b, Adj (&a)[NC],
                           const Globals& G) {
@@ -244,10 +369,14 @@ BG_HD void vjp_bend_exact(const Particle& p, const AdjCache& k, const double* __
   const double R = sqrt(pt2 - pxf * pxf), iR = 1 / R;
   const double Cp = ca * ps - sa * px;
   const double N = 2 * pxf + g_tot * h;
-  const bool fwd = Cp > 0;
-  const double iD = fwd ? 1 / (R + Cp) : 1 / g_tot;
-  const double xi = fwd ? h * N * iD : (R - Cp) * iD;
+  const double iD = 1 / (R + Cp);
+  const double xi = h * N * iD;
   const double Lv = h0 + x * sa;
+  if (!(l > 0 && fabs(b[4]) <= 1.5 && Cp > 0 && Lv > 0 && Cp * Lv + (pxf + g_tot * h) * xi > 0)) {  // NaN too
+#pragma unroll
+    for (int i = 0; i < NC; i++) vjp_bend_trig(p, b, a[i], G);
+    return;
+  }
   const double Lc = sqrt(xi * xi + Lv * Lv), iLc = 1 / Lc;
   const double s = 0.5 * g_tot * Lc * ipt, q = s * s;
   double F, dF;  // F and dF/dq
@@ -257,10 +386,7 @@ BG_HD void vjp_bend_exact(const Particle& p, const AdjCache& k, const double* __
     dF = 1.0 / 6 + q * (3.0 / 20 + q * (15.0 / 112 + q * (35.0 / 288 + q * (315.0 / 2816 + q * (693.0 / 6656 +
             q * (1001.0 / 10240))))));
   } else {
-    // half the bending angle, beyond a right angle where the chord shortens again
-    double hp = asin(fmin(fabs(s), 1.0));
-    const double ct = fwd ? 1.0 : Cp * Lv + (pxf + g_tot * h) * xi;  // sign of cos(angle + phi_1 - theta)
-    if (ct < 0) hp = kPi - hp;
+    const double hp = asin(fmin(fabs(s), 1.0));
     F = hp / fabs(s);
     dF = (1 / cos(hp) - F) / (2 * q);
   }
@@ -275,7 +401,7 @@ BG_HD void vjp_bend_exact(const Particle& p, const AdjCache& k, const double* __
     const double dpxf = ca * dpx + sa * d_ps[i] - g_tot * dh;
     const double dR = (d_pt2[i] - pxf * dpxf) * iR;
     const double dCp = ca * d_ps[i] - sa * dpx;
-    const double dxi = fwd ? (dh * N + h * (2 * dpxf + g_tot * dh) - xi * (dR + dCp)) * iD : (dR - dCp) * iD;
+    const double dxi = (dh * N + h * (2 * dpxf + g_tot * dh) - xi * (dR + dCp)) * iD;
     const double dLc = (xi * dxi + (i == 0 ? Lv * sa : 0.0)) * iLc;
     const double dpt = d_pt2[i] * ipt * ipt;  // over pt
     const double dLp = dLc * F + Lc * dF * (2 * q) * (dLc * iLc - dpt);
