@@ -88,7 +88,9 @@ __device__ __forceinline__ void get7(const double* q, int64_t stride, Particle& 
 
 // Turns [t0, t0 + n_t) of every particle that is alive, from its vec/beta (from_vec) or from turns row
 // row_in; before turn t (every `every`-th of the run) the state goes to turns row row0 + (t - t0) / every.
-// The state after the last turn returns to vec/beta/state when from_vec is set.
+// The state after the last turn returns to vec/beta/state when from_vec is set. REF: the reference's element
+// order, for lattices that track in it (Globals::hi_hot_pz = 0).
+template <bool REF>
 __global__ void __launch_bounds__(kAdjBlock) k_adj_forward(const __grid_constant__ AdjArgs a, int t0, int n_t, int every,
                                                            int row0, int row_in, int from_vec) {
   const int64_t j = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x;
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_forward(const __grid_constant
   bool alive = true;
   for (int t = 0; t < n_t && alive; ++t) {
     if (t % every == 0) put7(a.turns + (int64_t)(row0 + t / every) * 7 * N + j, N, p);
-    alive = track_turn<false>(p, a.hdr, a.pool, a.ap, a.G, 0, a.n_ele, t0 + t == 0, t0 + t, li);
+    alive = track_turn<false, REF>(p, a.hdr, a.pool, a.ap, a.G, 0, a.n_ele, t0 + t == 0, t0 + t, li);
   }
   if (!from_vec) return;
   a.vec[j] = p.x;
@@ -140,6 +142,7 @@ __global__ void k_adj_loss(const __grid_constant__ AdjArgs a) {
 }
 
 // Row row0 + t of turns is the start of the chunk's turn t; first: it is the run's first turn.
+template <bool REF>
 __global__ void __launch_bounds__(128) k_adj_inputs(const __grid_constant__ AdjArgs a, int row0, int first) {
   const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (i >= a.NT) return;
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(128) k_adj_inputs(const __grid_constant__ AdjA
   LossInfo li;
   for (int ie = 0; ie < a.n_ele; ++ie) {
     put7(a.inputs + (int64_t)ie * 7 * a.NT + i, a.NT, p);
-    track_turn<false>(p, a.hdr, a.pool, a.ap, a.G, ie, ie + 1, first && t == 0 && ie == 0, 0, li);
+    track_turn<false, REF>(p, a.hdr, a.pool, a.ap, a.G, ie, ie + 1, first && t == 0 && ie == 0, 0, li);
   }
 }
 
@@ -425,21 +428,29 @@ extern "C" int bmadgpu_loss_grad(bmadgpu_ctx* c, const bmadgpu_lattice* lat, con
   a.lossbuf = d_loss;
   a.loss_scale = 1.0 / (double)N;
   const unsigned grid = (unsigned)((N + kAdjBlock - 1) / kAdjBlock);
-  k_adj_forward<<<grid, kAdjBlock, 0, s>>>(a, 0, n_turns, whole ? 1 : seg, 0, 0, 1);
+#if defined(BG_FAST_MAPS)
+  const bool ref = a.G.hi_hot_pz == 0;
+  const auto forward = ref ? k_adj_forward<true> : k_adj_forward<false>;
+  const auto inputs = ref ? k_adj_inputs<true> : k_adj_inputs<false>;
+#else
+  const auto forward = k_adj_forward<false>;
+  const auto inputs = k_adj_inputs<false>;
+#endif
+  forward<<<grid, kAdjBlock, 0, s>>>(a, 0, n_turns, whole ? 1 : seg, 0, 0, 1);
   k_adj_loss<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(a);
   c->launches += 2;
   for (int32_t g = n_seg - 1; g >= 0; --g) {
     const int32_t t0 = g * seg, nt = std::min(seg, n_turns - t0);
     const int32_t row0 = whole ? 0 : n_seg;
     if (!whole) {
-      k_adj_forward<<<grid, kAdjBlock, 0, s>>>(a, t0, nt, 1, row0, g, 0);
+      forward<<<grid, kAdjBlock, 0, s>>>(a, t0, nt, 1, row0, g, 0);
       c->launches++;
     }
     for (int32_t end = nt; end > 0;) {
       const int32_t begin = std::max(0, end - chunk), n = end - begin;
       a.NT = (int64_t)n * N;
       const unsigned wide = (unsigned)((a.NT + 127) / 128);
-      k_adj_inputs<<<wide, 128, 0, s>>>(a, row0 + begin, t0 + begin == 0);
+      inputs<<<wide, 128, 0, s>>>(a, row0 + begin, t0 + begin == 0);
       k_adj_turnjac<<<wide, 128, 0, s>>>(a);
       k_adj_chain<<<grid, kAdjBlock, 0, s>>>(a, n);
       k_adj_grad<<<wide, 128, 0, s>>>(a);

@@ -3,9 +3,9 @@
 // k_batch_track: a persistent grid (one full wave of CTAs) pulls work items from a device
 // counter. An item is (variant, tile of `tile` consecutive entries of the variant's live list);
 // items of variant v are numbered tile_prefix[v] .. tile_prefix[v+1]-1. A CTA that moves to a
-// new variant takes up that variant's element table: the default build reads it from global memory
-// through L1, the correctly rounded one re-stages it into shared memory with a bulk copy (mbarrier
-// completion, bounded wait, the phase bit flipping on every use). Each thread tracks
+// new variant takes up that variant's element table: the element forms of the default build read it from
+// global memory through L1; the correctly rounded build, and lattices in the reference's order, re-stage it
+// into shared memory with a bulk copy (mbarrier completion, bounded wait, the phase bit flipping on every use). Each thread tracks
 // `ppt` particles of the tile one after another, each through all turns of the launch, with the
 // same per-particle code as k_track (particle.cuh). Survivors are appended to the variant's next
 // live list with a warp ballot and one atomic per warp, so compaction needs no extra pass.
@@ -14,6 +14,8 @@
 // the variants, reset of the work counter and of the next launch's live counts.
 
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "batch.cuh"
 #include "batch_kernel.cuh"
@@ -33,7 +35,8 @@ __global__ void k_batch_plan(const BatchVar* __restrict__ vars, int n_var, int t
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
   if (threadIdx.x == 0) {
     carry = 0;
-    *queue = 0;
+    queue[0] = 0;
+    queue[1] = 0;
   }
   __syncthreads();
   for (int base = 0; base < n_var; base += blockDim.x) {
@@ -90,8 +93,7 @@ struct Variant {
   const void* fn_lean;
 };
 #if defined(BG_FAST_MAPS)
-#define BG_BATCH_VARIANT(B, M) \
-  {B, M, (const void*)k_batch_track<B, M, false, true>, (const void*)k_batch_track<B, M, false, true>}
+#define BG_BATCH_VARIANT(B, M) {B, M, (const void*)k_batch_track<B, M, false, true>, nullptr}
 #else
 #define BG_BATCH_VARIANT(B, M) \
   {B, M, (const void*)k_batch_track<B, M, false, true>, (const void*)k_batch_track<B, M, false, false>}
@@ -102,6 +104,27 @@ const Variant kVariants[] = {
     BG_BATCH_VARIANT(256, 2), BG_BATCH_VARIANT(256, 3), BG_BATCH_VARIANT(512, 1),
 };
 #undef BG_BATCH_VARIANT
+#if defined(BG_FAST_MAPS)
+#define BG_SHAPE(B, M) {B, M, nullptr, nullptr}
+const Variant kRefShapes[] = {BG_REF_SHAPES(BG_SHAPE)};
+#undef BG_SHAPE
+#endif
+
+// Same register-budget selection as launch_track: the largest minimum CTA count not above ctas (0: the most
+// registers per thread), else the one with the most registers.
+template <int N>
+const Variant* pick(const Variant (&list)[N], int block, int ctas) {
+  const Variant* v = nullptr;
+  for (const Variant& k : list) {
+    if (k.block != block) continue;
+    if (ctas > 0 && k.minb > ctas) continue;
+    if (!v || (ctas > 0 ? k.minb > v->minb : k.minb < v->minb)) v = &k;
+  }
+  if (!v)
+    for (const Variant& k : list)
+      if (k.block == block && (!v || k.minb < v->minb)) v = &k;
+  return v;
+}
 
 }  // namespace
 
@@ -116,74 +139,83 @@ cudaError_t batch_upload_constants() {
 }
 
 cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_count, BatchKernel* out) {
-#if defined(BG_FAST_MAPS)
-  smem_bytes = 0;  // this build's kernels do not stage (batch_kernel.cuh)
-#endif
-  // same register-budget selection as launch_track
-  const Variant* v = nullptr;
-  for (const Variant& k : kVariants) {
-    if (k.block != cfg.block) continue;
-    if (cfg.ctas_per_sm > 0 && k.minb > cfg.ctas_per_sm) continue;
-    if (!v || (cfg.ctas_per_sm > 0 ? k.minb > v->minb : k.minb < v->minb)) v = &k;
-  }
-  // no variant compiled for so few CTAs per SM: the one with the most registers per thread
-  if (!v)
-    for (const Variant& k : kVariants)
-      if (k.block == cfg.block && (!v || k.minb < v->minb)) v = &k;
+  const Variant* v = pick(kVariants, cfg.block, cfg.ctas_per_sm);
   if (!v || cfg.particles_per_thread < 1) return cudaErrorInvalidValue;
-  cudaError_t err = cudaFuncSetAttribute(v->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  if (err != cudaSuccess) return err;
-  const void* fn_rec = batch_rec_kernel(v->block, v->minb);
-  if (!fn_rec) return cudaErrorInvalidValue;
-  err = cudaFuncSetAttribute(fn_rec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  if (err != cudaSuccess) return err;
-  int per_sm = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v->fn, cfg.block, smem_bytes);
-  if (err != cudaSuccess) return err;
-  if (per_sm < 1) per_sm = 1;
-  int per_sm_rec = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rec, fn_rec, cfg.block, smem_bytes);
-  if (err != cudaSuccess) return err;
-  if (per_sm_rec < 1) per_sm_rec = 1;
-  err = cudaFuncSetAttribute(v->fn_lean, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  if (err != cudaSuccess) return err;
-  int per_sm_lean = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_lean, v->fn_lean, cfg.block, smem_bytes);
-  if (err != cudaSuccess) return err;
-  if (per_sm_lean < 1) per_sm_lean = 1;
-  out->fn_lean = v->fn_lean;
-  out->grid_lean = sm_count * per_sm_lean;
-  const void* fn_rec_lean = batch_rec_kernel(v->block, v->minb, false);
-  if (!fn_rec_lean) return cudaErrorInvalidValue;
-  err = cudaFuncSetAttribute(fn_rec_lean, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-  if (err != cudaSuccess) return err;
-  int per_sm_rec_lean = 0;
-  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rec_lean, fn_rec_lean, cfg.block, smem_bytes);
-  if (err != cudaSuccess) return err;
-  if (per_sm_rec_lean < 1) per_sm_rec_lean = 1;
-  out->fn_rec_lean = fn_rec_lean;
-  out->grid_rec_lean = sm_count * per_sm_rec_lean;
-  out->fn = v->fn;
-  out->fn_rec = fn_rec;
-  out->grid_rec = sm_count * per_sm_rec;
+  *out = BatchKernel();
+  const void* fn[3][2];
+#if defined(BG_FAST_MAPS)
+  const Variant* m = pick(kRefShapes, cfg.block, cfg.ctas_per_sm);
+  if (!m) return cudaErrorInvalidValue;
+  fn[kBatchForms][0] = v->fn;
+  fn[kBatchForms][1] = batch_rec_kernel(v->block, v->minb);
+  for (int form : {kBatchFull, kBatchLean}) {
+    fn[form][0] = batch_ref_kernel(m->block, m->minb, form == kBatchFull);
+    fn[form][1] = batch_ref_rec_kernel(m->block, m->minb, form == kBatchFull);
+  }
+  const int first = kBatchForms;
+#else
+  for (int form : {kBatchFull, kBatchLean}) {
+    fn[form][0] = form == kBatchFull ? v->fn : v->fn_lean;
+    fn[form][1] = batch_rec_kernel(v->block, v->minb, form == kBatchFull);
+  }
+  const int first = kBatchFull;
+#endif
+  for (int form = first; form <= kBatchLean; form++)
+    for (int rec = 0; rec < 2; rec++) {
+      const void* f = fn[form][rec];
+      if (!f) return cudaErrorInvalidValue;
+      uint32_t smem = form == kBatchForms ? 0 : smem_bytes;
+      cudaError_t err = cudaSuccess;
+      // the same limit from every caller: servers and batches share these kernels
+      if (smem) err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxStageBytes);
+      if (err != cudaSuccess) return err;
+      int per_sm = 0;
+      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, cfg.block, smem);
+      if (err != cudaSuccess) return err;
+#if defined(BG_FAST_MAPS)
+      if (smem) {
+        int bare = 0;
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bare, f, cfg.block, 0);
+        if (err != cudaSuccess) return err;
+        if (per_sm < bare) {  // as much as leaves the resident CTAs as they are; larger tables go through L1
+          size_t room = 0;
+          err = cudaOccupancyAvailableDynamicSMemPerBlock(&room, f, bare, cfg.block);
+          if (err != cudaSuccess) return err;
+          smem = (uint32_t)std::min<size_t>(smem, room) & ~127u;
+          per_sm = bare;
+        }
+      }
+#endif
+      out->fn[form][rec] = f;
+      out->grid[form][rec] = sm_count * (per_sm < 1 ? 1 : per_sm);
+      out->smem[form][rec] = smem;
+    }
   out->block = cfg.block;
-  out->grid = sm_count * per_sm;
   out->ppt = cfg.particles_per_thread;
-  out->smem = smem_bytes;
   return cudaSuccess;
 }
 
-cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& a, cudaStream_t stream, bool record) {
+cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& args_in, cudaStream_t stream, bool record,
+                               int64_t* launches) {
+  BatchArgs a = args_in;
   int ppt = k.ppt;
   void* args[] = {(void*)&a, (void*)&ppt};
-  if (record && !a.rare)
-    return cudaLaunchKernel(k.fn_rec_lean, dim3((unsigned)k.grid_rec_lean), dim3((unsigned)k.block), args, k.smem,
-                            stream);
-  if (record)
-    return cudaLaunchKernel(k.fn_rec, dim3((unsigned)k.grid_rec), dim3((unsigned)k.block), args, k.smem, stream);
-  if (!a.rare)
-    return cudaLaunchKernel(k.fn_lean, dim3((unsigned)k.grid_lean), dim3((unsigned)k.block), args, k.smem, stream);
-  return cudaLaunchKernel(k.fn, dim3((unsigned)k.grid), dim3((unsigned)k.block), args, k.smem, stream);
+  const int inl = a.rare ? kBatchFull : kBatchLean;
+#if defined(BG_FAST_MAPS)
+  const int forms[2] = {a.ref < 2 ? (int)kBatchForms : -1, a.ref > 0 ? inl : -1};
+#else
+  a.ref = 0;
+  const int forms[2] = {inl, -1};
+#endif
+  for (int form : forms) {
+    if (form < 0) continue;
+    a.smem_bytes = k.smem[form][record];
+    cudaError_t err = cudaLaunchKernel(k.fn[form][record], dim3((unsigned)k.grid[form][record]),
+                                       dim3((unsigned)k.block), args, a.smem_bytes, stream);
+    if (err != cudaSuccess) return err;
+    (*launches)++;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t batch_launch_plan(const BatchVar* vars, int32_t n_var, int32_t tile, int32_t turn_off, bool identity,

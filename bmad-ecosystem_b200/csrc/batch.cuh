@@ -8,6 +8,8 @@
 
 namespace bmadgpu {
 
+constexpr uint32_t kMaxStageBytes = 200 * 1024;  // largest table staged in shared memory
+
 // Per-variant descriptor in device memory (one lattice + its particles).
 struct BatchVar {
   const uint8_t* table;       // packed element table
@@ -46,10 +48,13 @@ struct BatchArgs {
   const unsigned long long* n_in;    // [n_var] live-list lengths (unused with live_in == nullptr)
   int32_t* live_out;                 // nullptr: no compaction after this launch
   unsigned long long* n_out;         // [n_var] lengths of the compacted lists
-  unsigned long long* queue;         // work-item counter, zero at launch
+  unsigned long long* queue;         // [2] work-item counters, zero at launch (the second for REF kernels)
   int32_t* err_flag;                 // bit 0: table staging wait timed out
-  uint32_t smem_bytes;               // dynamic shared memory for staging (0: read tables from global)
+  uint32_t smem_bytes;               // dynamic shared memory for staging (0: read tables from global); set by
+                                     // batch_launch_track
   int32_t rare;                      // some variant's table has extra blocks / pitched offsets
+  int32_t ref;                       // variants that track in the reference's order (Globals::hi_hot_pz = 0):
+                                     // 0 none, 1 some, 2 all
 };
 
 struct BatchLaunch {
@@ -58,26 +63,35 @@ struct BatchLaunch {
   int particles_per_thread = 1;
 };
 
-// Kernel + grid of a launch shape (resolved once, outside stream capture).
+// Which instantiation a launch takes: the forms of fastmaps.cuh, or with the reference's element forms inline
+// for every element form (full) or for tables without rare ones (lean, TableInfo::rare).
+enum BatchForm : int { kBatchForms = 0, kBatchFull = 1, kBatchLean = 2 };
+
+// Kernels + grids of a launch shape (resolved once, outside stream capture).
 struct BatchKernel {
-  const void* fn = nullptr;
-  int block = 0, grid = 0, ppt = 1;
-  uint32_t smem = 0;
-  const void* fn_rec = nullptr;  // the same shape with the frequency-map record path
-  int grid_rec = 0;
-  const void* fn_lean = nullptr; // the same shape for tables without rare forms (TableInfo::rare)
-  int grid_lean = 0;
-  const void* fn_rec_lean = nullptr;
-  int grid_rec_lean = 0;
+  int block = 0, ppt = 1;
+  const void* fn[3][2] = {};     // [BatchForm][with the frequency-map record path]
+  int grid[3][2] = {};
+  uint32_t smem[3][2] = {};      // dynamic shared memory for staging tables
 };
 
 cudaError_t batch_upload_constants();
-cudaError_t batch_rec_upload_constants();            // batch_rec.cu's copy of the tables
-// record-path instantiation of a shape (full: every element form; else the lean one)
+// The other translation units' copies of the tables, and their instantiations of a shape: with the record
+// path (full: every element form, else the lean one), in the reference's order (default build; shapes of
+// BG_REF_SHAPES, else null), and with both.
+cudaError_t batch_rec_upload_constants();
+cudaError_t batch_ref_upload_constants();
+cudaError_t batch_ref_rec_upload_constants();
 const void* batch_rec_kernel(int block, int minb, bool full = true);
+const void* batch_ref_kernel(int block, int minb, bool full);
+const void* batch_ref_rec_kernel(int block, int minb, bool full);
+// smem_bytes: shared memory for staging, as much as the largest table that may be staged. The default build
+// takes it for lattices in the reference's order alone, and no more than leaves the resident CTAs unchanged.
 cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_count, BatchKernel* out);
-// record: use the instantiation with the frequency-map record path (rounds with an FMA job).
-cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& a, cudaStream_t stream, bool record = false);
+// record: use the instantiation with the frequency-map record path (rounds with an FMA job). *launches: kernels
+// launched.
+cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& a, cudaStream_t stream, bool record,
+                               int64_t* launches);
 // Work plan for a launch: tile_prefix from the live counts (or the variants' sizes when
 // identity is set), restricted to variants with turns left after turn_off; zeroes the queue
 // counter and the next launch's counts (n_zero, nullable).

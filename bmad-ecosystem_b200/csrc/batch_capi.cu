@@ -35,6 +35,7 @@ struct bmadgpu_batch {
   unsigned long long* d_queue = nullptr;
   uint32_t smem_bytes = 0;        // largest stageable table
   int32_t rare = 0;               // some variant's table has extra blocks / pitched offsets
+  int32_t ref = 0;                // variants in the reference's order: 0 none, 1 some, 2 all (BatchArgs::ref)
   bmadgpu_batch_tuning tuning;
   cudaGraphExec_t exec = nullptr;
   int32_t graph_turns = -1;
@@ -45,7 +46,6 @@ struct bmadgpu_batch {
 
 namespace {
 
-constexpr uint32_t kMaxStageBytes = 200 * 1024;
 
 size_t state_bytes(int64_t total) { return (size_t)total * (8 * sizeof(double) + 4 * sizeof(int32_t)); }
 
@@ -84,7 +84,6 @@ int resolve(bmadgpu_batch* b, BatchKernel* k) {
 // Enqueues the plan/track sequence of one call (n_turns > 0) on the context stream.
 int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64_t* launches) {
   const bmadgpu_batch_tuning& tu = b->tuning;
-  const uint32_t smem = k.smem;
   const int32_t tile = tu.block * tu.particles_per_thread;
   const int32_t tpl = tu.turns_per_launch > 0 ? std::min(tu.turns_per_launch, n_turns) : n_turns;
   const int32_t n_chunks = (n_turns + tpl - 1) / tpl;
@@ -106,8 +105,8 @@ int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64
   a.tile_prefix = b->d_prefix;
   a.queue = b->d_queue;
   a.err_flag = b->ctx->d_err;
-  a.smem_bytes = smem;
   a.rare = b->rare;
+  a.ref = b->ref;
   for (int32_t c = 0; c < n_chunks; ++c) {
     const bool last = c == n_chunks - 1;
     a.turn_off = c * tpl;
@@ -116,8 +115,7 @@ int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64
     a.n_in = c == 0 ? nullptr : b->d_cnt + (size_t)((c - 1) & 1) * b->n_var;
     a.live_out = last ? nullptr : b->d_live[c & 1];
     a.n_out = last ? nullptr : b->d_cnt + (size_t)(c & 1) * b->n_var;
-    CUDA_TRY(batch_launch_track(k, a, s));
-    (*launches)++;
+    CUDA_TRY(batch_launch_track(k, a, s, false, launches));
     if (!last) {
       CUDA_TRY(batch_launch_plan(b->d_vars, b->n_var, tile, (c + 1) * tpl, false, a.n_out, b->d_prefix, b->d_queue,
                                  b->d_cnt + (size_t)((c + 1) & 1) * b->n_var, s));
@@ -212,9 +210,11 @@ int bmadgpu_batch_create(bmadgpu_ctx* c, int32_t n_var, const bmadgpu_lattice* c
   b->offs.resize(n_var);
   std::vector<BatchVar> hv(n_var);
   int64_t off = 0;
+  int32_t n_ref = 0;
   for (int32_t v = 0; v < n_var; ++v) {
     const bmadgpu_lattice* L = lats[v];
     if (L->pk.info.rare) b->rare = 1;
+    n_ref += L->G.hi_hot_pz == 0;
     b->offs[v] = off;
     BatchVar& d = hv[v];
     std::memset(&d, 0, sizeof(d));
@@ -227,22 +227,31 @@ int bmadgpu_batch_create(bmadgpu_ctx* c, int32_t n_var, const bmadgpu_lattice* c
     d.ap_bytes = L->pk.info.ap_bytes;
     d.n_ele = L->pk.info.n_ele;
     d.G = L->G;
-    if (d.table_bytes <= kMaxStageBytes) b->smem_bytes = std::max(b->smem_bytes, d.table_bytes);
+#if defined(BG_CR_MATH)
+    const bool staged = d.table_bytes <= kMaxStageBytes;
+#else
+    const bool staged = d.table_bytes <= kMaxStageBytes && d.G.hi_hot_pz == 0;  // the others are read through L1
+#endif
+    if (staged) b->smem_bytes = std::max(b->smem_bytes, d.table_bytes);
     off += counts[v];
   }
+  b->ref = n_ref == 0 ? 0 : n_ref < n_var ? 1 : 2;
   const size_t T = (size_t)std::max<int64_t>(total, 1);
   b->tuning = bmadgpu_batch_tuning{128, 0, 1, 0, 1, 1, {0, 0}};
 #if !defined(BG_CR_MATH)
   // As the plain kernel's rule (track.cu, shape_for), but 16 warps per SM at 128 registers up to two waves
   // of them, since the work queue evens out the second one: 130k particles of 24 rings, 8 turns, 3.7 ms
-  // against 4.4 with 24 warps at 80 registers; 390k particles 11.4 against 10.5.
+  // against 4.4 with 24 warps at 80 registers; 390k particles 11.4 against 10.5. The reference's element
+  // order needs more registers (128 x 3, 168): a batch of lattices in that order keeps them.
   const int64_t row = (int64_t)64 * c->sm_count;
-  if (total <= 8 * row) {
-    b->tuning.block = 64;
-    b->tuning.ctas_per_sm = total <= 4 * row ? 4 : 8;
-  } else {
-    b->tuning.block = total <= 16 * row ? 128 : 256;
-    b->tuning.ctas_per_sm = total <= 16 * row ? 4 : 3;
+  if (b->ref < 2) {
+    if (total <= 8 * row) {
+      b->tuning.block = 64;
+      b->tuning.ctas_per_sm = total <= 4 * row ? 4 : 8;
+    } else {
+      b->tuning.block = total <= 16 * row ? 128 : 256;
+      b->tuning.ctas_per_sm = total <= 16 * row ? 4 : 3;
+    }
   }
 #endif
   if (cudaMalloc(&b->d_vars, sizeof(BatchVar) * n_var) != cudaSuccess ||
@@ -254,7 +263,7 @@ int bmadgpu_batch_create(bmadgpu_ctx* c, int32_t n_var, const bmadgpu_lattice* c
       cudaMalloc(&b->d_live[1], T * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_cnt, 2 * sizeof(unsigned long long) * n_var) != cudaSuccess ||
       cudaMalloc(&b->d_prefix, sizeof(int64_t) * (n_var + 1)) != cudaSuccess ||
-      cudaMalloc(&b->d_queue, sizeof(unsigned long long)) != cudaSuccess) {
+      cudaMalloc(&b->d_queue, 2 * sizeof(unsigned long long)) != cudaSuccess) {
     bmadgpu_batch_destroy(b);
     return fail(BMADGPU_ENOMEM, "cannot allocate the batch's device state");
   }

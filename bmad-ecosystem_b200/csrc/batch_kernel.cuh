@@ -9,6 +9,10 @@
 #include "tma.cuh"
 #include "track.cuh"
 
+// Launch shapes (threads per CTA, CTAs per SM) of the REF instantiations: every block size, the register
+// budgets 255, 168, 128 and 85.
+#define BG_REF_SHAPES(V) V(64, 4), V(64, 8), V(128, 3), V(128, 4), V(128, 6), V(256, 2), V(512, 1)
+
 namespace bmadgpu {
 
 namespace {
@@ -36,8 +40,12 @@ __device__ __noinline__ void fma_record(const BatchVar& v, int64_t j, int32_t t_
 }
 
 // REC: the instantiation for rounds that hold a frequency-map job; every other launch uses the
-// REC = false code, which has no record path at all.
-template <int BLOCK, int MINB, bool REC, bool FULL = true>
+// REC = false code, which has no record path at all. REF (default build): the reference's element order inline,
+// for the lattices that track in it (Globals::hi_hot_pz = 0), where with the forms of fastmaps.cuh each of
+// their elements is an out-of-line call (4096 particles of a ring with thin multipoles between its elements,
+// 4 turns: 10.6 ms against 6.4). A launch that holds lattices of both sorts is one of each kernel, which
+// leave each other's work items alone (a.ref == 1).
+template <int BLOCK, int MINB, bool REC, bool FULL = true, bool REF = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_constant__ BatchArgs a, int ppt) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bar;
@@ -45,9 +53,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
   __shared__ long long s_item;
   __shared__ int s_var;
 #if defined(BG_FAST_MAPS)
-  // Tables are read from global memory through L1: with loads known to be global it takes 1 % longer than
-  // from shared memory on a small ring's table, and a staged table of the larger ones costs residency.
-  bool can_stage = false;
+  // The forms read their tables from global memory through L1: with loads known to be global it takes 1 %
+  // longer than from shared memory on a small ring's table, and a staged table of the larger ones costs
+  // residency.
+  bool can_stage = REF && a.smem_bytes > 0;
 #else
   bool can_stage = a.smem_bytes > 0;
 #endif
@@ -61,9 +70,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
 
   for (;;) {
     if (threadIdx.x == 0) {
-      const long long item = (long long)atomicAdd(a.queue, 1ull);
-      int v = -1;
-      if (item < total) {
+      long long item;
+      int v;
+      for (;;) {
+        item = (long long)atomicAdd(a.queue + REF, 1ull);
+        v = -1;
+        if (item >= total) break;
         // last variant whose first item is <= item (variants without items share their
         // successor's prefix value and are skipped)
         int lo = 0, hi = a.n_var - 1;
@@ -73,6 +85,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
           else hi = mid - 1;
         }
         v = lo;
+        if (a.ref != 1 || (a.vars[v].G.hi_hot_pz == 0) == REF) break;
       }
       s_item = item;
       s_var = v;
@@ -102,8 +115,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
     }
 
 #if defined(BG_FAST_MAPS)
-    tbl = sv.table;
-    __builtin_assume(__isGlobal(tbl));
+    if (!REF) {
+      tbl = sv.table;
+      __builtin_assume(__isGlobal(tbl));
+    }
 #endif
     const EleHdr* hdr = reinterpret_cast<const EleHdr*>(tbl);
     const ApRec* ap = reinterpret_cast<const ApRec*>(tbl + sv.hdr_bytes);
@@ -131,9 +146,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
       const double z_in = p.z, beta_in = p.beta;
       LossInfo li;
       if (alive) {
-        refresh_particle(p, G);
+        if (REF) refresh(p, G);
+        else refresh_particle(p, G);
         for (int turn = 0; turn < nt && alive; ++turn) {
-          alive = track_turn<FULL>(p, hdr, pool, ap, G, 0, n_ele, turn == 0, turn_no0 + turn, li);
+          alive = track_turn<FULL, REF>(p, hdr, pool, ap, G, 0, n_ele, turn == 0, turn_no0 + turn, li);
           if (REC && sv.rec && alive)
             fma_record(sv, j, turn_no0 + turn - sv.rec_turn0, p.x, p.px, p.y, p.py, p.z, p.pz);
         }

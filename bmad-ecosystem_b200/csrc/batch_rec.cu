@@ -15,7 +15,7 @@ const void* batch_rec_kernel(int block, int minb, bool full) {
     const void* fn_lean;
   };
 #if defined(BG_FAST_MAPS)
-#define BG_BATCH_REC(B, M) {B, M, (const void*)k_batch_track<B, M, true, true>, (const void*)k_batch_track<B, M, true, true>}
+#define BG_BATCH_REC(B, M) {B, M, (const void*)k_batch_track<B, M, true, true>, nullptr}
 #else
 #define BG_BATCH_REC(B, M) {B, M, (const void*)k_batch_track<B, M, true, true>, (const void*)k_batch_track<B, M, true, false>}
 #endif

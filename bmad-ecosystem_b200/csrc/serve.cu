@@ -161,7 +161,6 @@ struct bmadgpu_server {
   BatchVar* h_vars[kRoundsInFlight] = {nullptr, nullptr};
   unsigned long long* h_cnt[kRoundsInFlight] = {nullptr, nullptr};
   BatchKernel kern;
-  uint32_t smem = 0;
   // record arena for frequency-map jobs (doubles)
   double* d_rec = nullptr;
   int64_t rec_capacity = 0;
@@ -384,7 +383,7 @@ void worker_main(bmadgpu_server* s) {
     int32_t n_var = 0;
     std::vector<int64_t> round_jobs;
     bool round_records = false;
-    int32_t round_rare = 0;
+    int32_t round_rare = 0, round_ref = 0;  // round_ref: jobs of the round in the reference's order
     for (int32_t slot = 0; slot < (int32_t)s->slot_job.size(); ++slot) {
       const int64_t id = s->slot_job[slot];
       BatchVar& hv = s->h_vars[buf][slot];
@@ -405,6 +404,7 @@ void worker_main(bmadgpu_server* s) {
       j.last_round = r;
       round_jobs.push_back(id);
       round_records = round_records || j.fma;
+      round_ref += j.lat->G.hi_hot_pz == 0;
     }
     const bool stopping = s->stop;
     lk.unlock();
@@ -449,8 +449,9 @@ void worker_main(bmadgpu_server* s) {
       a.n_out = s->d_cnt + (size_t)(1 - parity) * J;
       a.queue = s->d_queue;
       a.err_flag = s->ctx->d_err;
-      a.smem_bytes = s->smem;
       a.rare = round_rare;
+      a.ref = round_ref == 0 ? 0 : round_ref < (int32_t)round_jobs.size() ? 1 : 2;
+      int64_t launched = 0;
       Round rd;
       rd.index = r;
       rd.parity = parity;
@@ -462,7 +463,7 @@ void worker_main(bmadgpu_server* s) {
                cudaSuccess &&
            batch_launch_plan(s->d_vars, n_var, a.tile, 0, false, a.n_in, s->d_prefix, s->d_queue, a.n_out, c) ==
                cudaSuccess &&
-           batch_launch_track(s->kern, a, c, round_records) == cudaSuccess &&
+           batch_launch_track(s->kern, a, c, round_records, &launched) == cudaSuccess &&
            cudaMemcpyAsync(s->h_cnt[buf], a.n_out, sizeof(unsigned long long) * n_var, cudaMemcpyDeviceToHost, c) ==
                cudaSuccess &&
            cudaEventRecord(rd.t1, c) == cudaSuccess &&
@@ -658,7 +659,7 @@ int bmadgpu_server_create(bmadgpu_ctx* c, const bmadgpu_server_config* cfg_in, b
             cudaMalloc(&s->d_vars, J * sizeof(BatchVar)) == cudaSuccess &&
             cudaMalloc(&s->d_cnt, 2 * J * sizeof(unsigned long long)) == cudaSuccess &&
             cudaMalloc(&s->d_prefix, (J + 1) * sizeof(int64_t)) == cudaSuccess &&
-            cudaMalloc(&s->d_queue, sizeof(unsigned long long)) == cudaSuccess;
+            cudaMalloc(&s->d_queue, 2 * sizeof(unsigned long long)) == cudaSuccess;
   for (int i = 0; ok && i < kRoundsInFlight; ++i)
     ok = cudaHostAlloc(&s->h_vars[i], J * sizeof(BatchVar), cudaHostAllocPortable) == cudaSuccess &&
          cudaHostAlloc(&s->h_cnt[i], J * sizeof(unsigned long long), cudaHostAllocPortable) == cudaSuccess;
@@ -678,12 +679,11 @@ int bmadgpu_server_create(bmadgpu_ctx* c, const bmadgpu_server_config* cfg_in, b
     }
   }
   if (ok) {
-    s->smem = cfg.stage_smem ? kServeStageBytes : 0;
     BatchLaunch bl;
     bl.block = cfg.block;
     bl.ctas_per_sm = cfg.ctas_per_sm;
     bl.particles_per_thread = 1;
-    ok = batch_resolve(bl, s->smem, c->sm_count, &s->kern) == cudaSuccess;
+    ok = batch_resolve(bl, cfg.stage_smem ? kServeStageBytes : 0, c->sm_count, &s->kern) == cudaSuccess;
   }
   if (!ok) {
     bmadgpu_server_destroy(s);

@@ -189,6 +189,10 @@ cudaError_t upload_constants() {
   if (e != cudaSuccess) return e;
   e = batch_rec_upload_constants();
   if (e != cudaSuccess) return e;
+  e = batch_ref_upload_constants();
+  if (e != cudaSuccess) return e;
+  e = batch_ref_rec_upload_constants();
+  if (e != cudaSuccess) return e;
   return adjoint_upload_constants();
 }
 
@@ -202,11 +206,13 @@ struct Variant {
 #if defined(BG_FAST_MAPS)
 #define BG_KERNELS(B, M) {(const void*)k_track<B, M, true, kGlobal>, (const void*)k_track<B, M, true, kShared>}
 #define BG_VARIANT(B, M) {B, M, BG_KERNELS(B, M), BG_KERNELS(B, M)}
-// For TrackArgs::ref: one warp's latency (up to four 64-thread CTAs per SM), and the whole chip.
+// For TrackArgs::ref: every block size, the register budgets 255, 168 and 128.
 #define BG_REF(B, M) \
   {B, M, {(const void*)k_track<B, M, true, kEither, true>, (const void*)k_track<B, M, true, kEither, true>}, \
    {(const void*)k_track<B, M, false, kEither, true>, (const void*)k_track<B, M, false, kEither, true>}}
-static const Variant kRefVariants[2] = {BG_REF(64, 4), BG_REF(256, 2)};
+static const Variant kRefVariants[] = {
+    BG_REF(64, 4), BG_REF(64, 8), BG_REF(128, 3), BG_REF(128, 4), BG_REF(256, 2), BG_REF(512, 1),
+};
 #undef BG_REF
 static const Variant kVariants[] = {
     BG_VARIANT(64, 4),  BG_VARIANT(64, 8),  BG_VARIANT(64, 12), BG_VARIANT(128, 4), BG_VARIANT(128, 6),
@@ -229,38 +235,46 @@ static const Variant kVariants[] = {
 // register budget without spills, and small CTAs so that all SMs get some (10,000 particles, 50-cell
 // ring: 0.16 ms a turn against 0.20 with 80 registers). A bunch that fills the chip wants the warps:
 // 24 per SM at 80 registers (1M particles, 200-cell ring: 16.4 ms a turn against 19.9 with 16 warps at
-// 128 registers and 27.2 with 8 at 255).
-static void shape_for(int64_t n, int sm_count, LaunchCfg* cfg) {
+// 128 registers and 27.2 with 8 at 255). The reference's element order needs more registers: 256 x 2 there.
+static void shape_for(int64_t n, int sm_count, bool ref, LaunchCfg* cfg) {
   const int64_t row = (int64_t)64 * sm_count;  // one 64-thread CTA on every SM
+  if (ref) {
+    cfg->block = n <= 4 * row ? 64 : 256;
+    cfg->ctas_per_sm = n <= 4 * row ? 4 : 2;
+    return;
+  }
   cfg->block = n <= 8 * row ? 64 : 256;
   cfg->ctas_per_sm = n <= 4 * row ? 4 : n <= 8 * row ? 8 : 3;
 }
 #endif
 
-cudaError_t launch_track(const TrackArgs& args_in, const LaunchCfg& cfg_in, int sm_count, cudaStream_t stream) {
-  TrackArgs a = args_in;
-  LaunchCfg cfg = cfg_in;
-#if defined(BG_FAST_MAPS)
-  if (cfg.automatic) shape_for(a.ld, sm_count, &cfg);
-  const Variant* ref = a.ref ? &kRefVariants[a.ld <= (int64_t)256 * sm_count ? 0 : 1] : nullptr;
-  if (ref) cfg.block = ref->block;
-#endif
-  int stage = (cfg.stage_smem && table_fits_smem(a.table_bytes)) ? 1 : 0;
-  // ctas_per_sm selects the register budget: the variant with the largest minimum CTA count
-  // not above it (0: the most registers per thread)
+// The variant of cfg's block whose minimum CTA count is the largest not above ctas_per_sm (0: the one with
+// the most registers per thread); where none is compiled for so few CTAs per SM, the one with the most
+// registers.
+template <int N>
+static const Variant* pick(const Variant (&list)[N], const LaunchCfg& cfg) {
   const Variant* v = nullptr;
-  for (const Variant& k : kVariants) {
+  for (const Variant& k : list) {
     if (k.block != cfg.block) continue;
     if (cfg.ctas_per_sm > 0 && k.minb > cfg.ctas_per_sm) continue;
     if (!v || (cfg.ctas_per_sm > 0 ? k.minb > v->minb : k.minb < v->minb)) v = &k;
   }
-  // no variant compiled for so few CTAs per SM: the one with the most registers per thread
   if (!v)
-    for (const Variant& k : kVariants)
+    for (const Variant& k : list)
       if (k.block == cfg.block && (!v || k.minb < v->minb)) v = &k;
+  return v;
+}
+
+cudaError_t launch_track(const TrackArgs& args_in, const LaunchCfg& cfg_in, int sm_count, cudaStream_t stream) {
+  TrackArgs a = args_in;
+  LaunchCfg cfg = cfg_in;
 #if defined(BG_FAST_MAPS)
-  if (ref) v = ref;
+  if (cfg.automatic) shape_for(a.ld, sm_count, a.ref, &cfg);
+  const Variant* v = a.ref ? pick(kRefVariants, cfg) : pick(kVariants, cfg);
+#else
+  const Variant* v = pick(kVariants, cfg);
 #endif
+  int stage = (cfg.stage_smem && table_fits_smem(a.table_bytes)) ? 1 : 0;
   if (!v) return cudaErrorInvalidValue;
   const void* const* fns = a.rare ? v->fn : v->fn_lean;
   int per_sm = 0;
