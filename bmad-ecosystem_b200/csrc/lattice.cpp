@@ -574,11 +574,13 @@ std::vector<double> bend_frame_block(const bmadgpu_element& e) {
   return blk;
 }
 
+#if defined(BG_TABLE_FORMS)
 // A bend's entries from SB_F and what they were made from (push_bend_series).
 struct BendSeries {
   double step_len = 0, g = 0, g_tot = 0;
   std::vector<double> v;
 };
+#endif
 
 struct Packer {
   std::vector<EleHdr> hdr;
@@ -586,7 +588,9 @@ struct Packer {
   std::vector<double> pool;
   std::map<std::vector<double>, uint32_t> dedupe;
   std::map<std::vector<double>, uint16_t> ap_dedupe;
+#if defined(BG_TABLE_FORMS)
   BendSeries bend;
+#endif
 
   uint32_t add_block(const std::vector<double>& blk) {
     if (blk.empty()) return 0;
@@ -611,6 +615,7 @@ struct Packer {
   }
 };
 
+#if defined(BG_TABLE_FORMS)
 // The frame block (table.h) of a pitched misalign block (straight) or a bend frame: the position
 // transforms of offset_particle's set and unset composed into one affine map of (x, y) each.
 std::vector<double> frame_block(const std::vector<double>& mis, bool straight) {
@@ -781,6 +786,7 @@ void push_bend_series(std::vector<double>& blk, double step_len, double g, doubl
   last.g_tot = g_tot;
   last.v.assign(blk.begin() + at, blk.end());
 }
+#endif  // BG_TABLE_FORMS
 
 void push_kicks(std::vector<double>& blk, const double* a, const double* b, int n_pole, double scale) {
   for (int n = 0; n < n_pole; n++) {
@@ -1107,7 +1113,9 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
             double cdpx = gt * ge * (1 + 2 * (tan_e * tan_e));
             blk.insert(blk.end(), {gt, gt2, gs2, k1_tane, fg_factor, ge, cdpx});
           }
+#if defined(BG_TABLE_FORMS)
           push_bend_series(blk, step_len, g, g_tot, pk.bend);
+#endif
           if (e.fringe_type == BMADGPU_FRINGE_BASIC_BEND || e.fringe_type == BMADGPU_FRINGE_HARD_EDGE_ONLY) {
             if (e.fringe_at == BMADGPU_ENTRANCE_END || e.fringe_at == BMADGPU_BOTH_ENDS) flags |= F_EDGE_IN;
             if (e.fringe_at == BMADGPU_EXIT_END || e.fringe_at == BMADGPU_BOTH_ENDS) flags |= F_EDGE_OUT;
@@ -1188,10 +1196,12 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
       }
       h.flags = flags;
       h.param = pk.add_block(blk);
+#if defined(BG_TABLE_FORMS)
       // a frame where there is no extra block: EleHdr::extra names it
       if ((flags & F_PITCH) && !(flags & F_EXTRA)) h.extra = pk.add_block(frame_block(mis, h.kind != K_SBEND));
       h.fast = fast_header(h, flags, blk, (flags & (F_AP_ENTRANCE | F_AP_EXIT)) ? &pk.ap[h.ap_index] : nullptr,
                            p.max_aperture_limit);
+#endif
       out.n_step[i] = h.n_step;
       pk.hdr.push_back(h);
     }
@@ -1215,8 +1225,10 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
     if (ti.ap_bytes) std::memcpy(out.image.data() + ti.hdr_bytes, pk.ap.data(), ti.ap_bytes);
     std::memcpy(out.image.data() + ti.hdr_bytes + ti.ap_bytes, pk.pool.data(), pk.pool.size() * sizeof(double));
     out.cold_prefix.assign(n_ele + 1, 0);
+#if defined(BG_TABLE_FORMS)
     for (int i = 0; i < n_ele; i++)
       out.cold_prefix[i + 1] = out.cold_prefix[i] + ((pk.hdr[i].fast.code & FC_BODY) == FC_COLD);
+#endif
     out.ref_time_prefix.assign(n_ele + 1, 0.0);
     for (int i = 0; i < n_ele; i++) out.ref_time_prefix[i + 1] = out.ref_time_prefix[i] + eles[i].delta_ref_time;
     return BMADGPU_OK;

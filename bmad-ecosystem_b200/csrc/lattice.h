@@ -14,7 +14,7 @@ struct PackedLattice {
   std::vector<int> n_step;             // resolved integration steps per element
   std::vector<double> ds_step;         // resolved ds_step per element
   std::vector<double> ref_time_prefix; // sum of delta_ref_time over elements [0, i)
-  std::vector<int32_t> cold_prefix;  // [n_ele + 1]: elements < i without a form in fastmaps.cuh
+  std::vector<int32_t> cold_prefix;  // [n_ele + 1]: elements < i without a form in fastmaps.cuh (default build)
 };
 
 int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p, PackedLattice& out,

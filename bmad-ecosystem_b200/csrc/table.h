@@ -43,6 +43,14 @@ enum Flag : uint16_t {
   F_AP_WINDOW = 1 << 15    // the aperture record carries collimator phase-space windows
 };
 
+// The entries that only the forms of fastmaps.cuh read (FastHdr, the bends' from SB_F, the frame blocks of
+// elements without an extra block) are left out of the correctly rounded build's tables, which its kernels
+// stage in shared memory: with them the residency of a large batch fell (24 rings of 1801 elements, 98,304
+// particles, 2 turns: 56 ms against 43).
+#if !defined(BG_CR_MATH)
+#define BG_TABLE_FORMS 1
+#endif
+
 // FastHdr::code: the element's form in fastmaps.cuh and what goes with it.
 enum FastCode : uint32_t {
   FC_COLD = 0,             // none
@@ -71,7 +79,7 @@ struct FastHdr {           // 16 bytes
   uint32_t acc_x, acc_y;
 };
 
-struct EleHdr {            // 32 bytes
+struct EleHdr {            // 32 bytes (16 without the forms' entries)
   uint8_t kind;
   uint8_t n_pole;          // number of multipole orders kicked (ix_mag_max + 1), 0 = none
   uint16_t flags;
@@ -79,7 +87,9 @@ struct EleHdr {            // 32 bytes
   uint16_t ap_index;       // index into the aperture records
   uint32_t param;          // offset (in doubles) of the parameter block in the pool
   uint32_t extra;          // offset (in doubles) of the extra block (F_EXTRA) or the frame block (F_PITCH), else 0
+#if defined(BG_TABLE_FORMS)
   FastHdr fast;
+#endif
 };
 
 struct ApRec {             // 112 bytes
@@ -141,7 +151,12 @@ struct ApRec {             // 112 bytes
 //           longitudinal fringe, EX_HARD hard_multipole_edge_kick, EX_SOFT
 //           soft_quadrupole_edge_kick, EX_EXACT exact_bend_edge_kick (in place of Hwang's), EX_ESEP
 //           the elseparator's longitudinal fringe.
-constexpr int SB_EDGE_IN = 12, SB_EDGE_OUT = 19, SB_F = 26, SB_FIXED = 46, QD_FIXED = 5, TH_FIXED = 2;
+constexpr int SB_EDGE_IN = 12, SB_EDGE_OUT = 19, SB_F = 26, QD_FIXED = 5, TH_FIXED = 2;
+#if defined(BG_TABLE_FORMS)
+constexpr int SB_FIXED = SB_F + 20;
+#else
+constexpr int SB_FIXED = SB_F;
+#endif
 #if defined(__CUDACC__)
 #define BG_TABLE_FN __host__ __device__
 #else
