@@ -85,7 +85,7 @@ constexpr uint32_t kHiNano = 0x3e112e0cu;     // one above that of 1e-9
 BG_HD uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
 // The cached functions of pz and beta for these maps; hot: the maps below cover this pz and beta
-// (|pz| < 1/4, not NaN), and the lattice has more elements with a form than without (Globals::hi_hot_pz).
+// (|pz| < 1/4, not NaN), and enough of the lattice's elements have a form (Globals::hi_hot_pz).
 // They change only in cold_track1.
 BG_HD void finish_f(Particle& p, const Globals& G) {  // from refresh()'s
   p.lez = p.lez_series ? p.pz * p.lez_a * G.lez_me2 : p.lez_a * G.inv_beta0;

@@ -191,7 +191,7 @@ struct Globals {            // branch constants (lat_param_struct / bmad_com) an
   double inv_beta0;         // 1 / beta0 (rounded), the shared reciprocal of the quotients by beta0
   uint32_t hi_max_ap;       // high word of max_ap (accepts a coordinate inside it, fastmaps.cuh)
   // high word of 1/4: particles with a smaller |pz| take the forms of fastmaps.cuh; 0 for a lattice with
-  // more elements without a form than with one, which tracks in the reference's forms throughout
+  // more than a third of its elements without one, which tracks in the reference's forms throughout
   uint32_t hi_hot_pz;
 };
 
