@@ -89,7 +89,7 @@ namespace bmadgpu {
 
 // Core device-side tracking: all bunch pointers are device pointers.
 int track_device(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bunch* b, int32_t ix_start,
-                 int32_t ix_end, int32_t turn0, int32_t n_turns, double* d_moments) {
+                 int32_t ix_end, int32_t turn0, int32_t n_turns, double* d_moments, bool ref) {
   if (b->n == 0 || n_turns == 0) return BMADGPU_OK;
   const bmadgpu_tuning& tu = c->tuning;
   int per_launch = tu.turns_per_launch > 0 ? tu.turns_per_launch : n_turns;
@@ -107,7 +107,7 @@ int track_device(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bunch
   a.table = lat->d_table;
   a.table_bytes = lat->pk.info.total_bytes;
   a.rare = (int32_t)lat->pk.info.rare;
-  a.ref = c->ref_forms || lat->G.hi_hot_pz == 0 ||
+  a.ref = ref || lat->G.hi_hot_pz == 0 ||
           lat->pk.cold_prefix[ix_end] - lat->pk.cold_prefix[ix_start] == ix_end - ix_start;
   a.hdr_bytes = lat->pk.info.hdr_bytes;
   a.ap_bytes = lat->pk.info.ap_bytes;

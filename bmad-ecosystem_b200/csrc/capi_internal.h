@@ -19,9 +19,9 @@ Globals make_globals(const bmadgpu_param& p);
 int check_err_flag(bmadgpu_ctx* c);
 // Enqueues n_turns of tracking of a device-resident bunch on the context stream with the
 // context's tuning (chunks of turns_per_launch, live-list compaction between them); d_moments,
-// if not NULL, receives the per-turn sums [n_turns][28].
+// if not NULL, receives the per-turn sums [n_turns][28]. ref: in the reference's element order (TrackArgs::ref).
 int track_device(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bunch* b, int32_t ix_start,
-                 int32_t ix_end, int32_t turn0, int32_t n_turns, double* d_moments);
+                 int32_t ix_end, int32_t turn0, int32_t n_turns, double* d_moments, bool ref = false);
 // Frequency-map tunes of n particles from their record hist [6][n_turn][n] (fma.cu): fstate[i]
 // = 1 where state[i] is not alive, else rec_state[i]; tunes [n][6] where fstate is 0.
 cudaError_t fma_launch_tunes(const double* hist, int64_t n, int32_t n_turn, int32_t N, const int32_t* state,
@@ -51,7 +51,6 @@ struct bmadgpu_ctx {
   double* d_mom = nullptr;
   int64_t mom_cap = 0;
   int32_t* d_i32 = nullptr;       // state, ix_ele, ix_turn, location: 4 * cap
-  int32_t ref_forms = 0;          // track_device: the reference's element forms (TrackArgs::ref)
   bool tuned = false;             // tuning was set by the caller or the autotuner
   bmadgpu_tuning tuning;
   int64_t launches = 0;           // kernel launches enqueued

@@ -196,7 +196,7 @@ double init_beta(const bmadgpu_param& p, double pz) {
 
 // One turn of the 25 stencil particles about x: f(x) and the one-turn matrix. *lost is set when
 // any of them is lost (the caller's cue to step back: the matrix needs all 25). ref: with the
-// reference's element forms, whose last bits f(x) then has (the caller reports it as the orbit).
+// reference's element forms, whose last bits f(x) and the matrix then have (bmadgpu_one_turn_matrix).
 int one_turn(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const double* x, double* fx, double* M,
              OrbitParticles& op, bool* lost, bool ref = false) {
   const int n = kStencil;
@@ -211,9 +211,7 @@ int one_turn(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const double* x, double
   CUDA_TRY(cudaMemcpyAsync(op.b.vec, op.hv.data(), sizeof(double) * 6 * n, cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(op.b.beta, op.hb.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(op.b.state, op.hs.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
-  c->ref_forms = ref;
-  int r = track_device(c, lat, &op.b, 0, (int32_t)lat->pk.info.n_ele, 0, 1, nullptr);
-  c->ref_forms = 0;
+  int r = track_device(c, lat, &op.b, 0, (int32_t)lat->pk.info.n_ele, 0, 1, nullptr, ref);
   if (r) return r;
   CUDA_TRY(cudaMemcpyAsync(op.hv.data(), op.b.vec, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaMemcpyAsync(op.hs.data(), op.b.state, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s));
@@ -391,7 +389,7 @@ extern "C" int bmadgpu_one_turn_matrix(bmadgpu_ctx* c, const bmadgpu_lattice* la
   if ((r = op.init())) return r;
   double fx[6];
   bool lost = false;
-  if ((r = one_turn(c, tmp.lat, orbit, fx, mat, op, &lost, orbit_end != nullptr))) return r;
+  if ((r = one_turn(c, tmp.lat, orbit, fx, mat, op, &lost, true))) return r;
   if (lost) return fail(BMADGPU_EINVAL, "the orbit particle or one of its stencil neighbours was lost in one turn");
   if (orbit_end) std::memcpy(orbit_end, fx, sizeof(fx));
   return BMADGPU_OK;
