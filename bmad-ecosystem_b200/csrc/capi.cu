@@ -128,7 +128,7 @@ int track_device(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bunch
   cfg.block = tu.block;
   cfg.ctas_per_sm = tu.ctas_per_sm;
   cfg.stage_smem = tu.stage_smem != 0;
-  cfg.automatic = !c->tuned;
+  cfg.automatic = tu.reserved[0] == 1;
   int cur = 0;  // which live list / count is current; live == nullptr means identity
   const int32_t* live = nullptr;
   for (int32_t done = 0; done < n_turns; done += per_launch) {
@@ -222,7 +222,7 @@ int noalloc_prepare(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_bu
   cfg->block = c->tuning.block;
   cfg->ctas_per_sm = c->tuning.ctas_per_sm;
   cfg->stage_smem = c->tuning.stage_smem != 0;
-  cfg->automatic = !c->tuned;
+  cfg->automatic = c->tuning.reserved[0] == 1;
   *sm_count = c->sm_count;
   *stream = c->stream;
   *launches = &c->launches;
@@ -275,7 +275,7 @@ int bmadgpu_ctx_create(int32_t device, bmadgpu_ctx** out) {
   if (!c) return fail(BMADGPU_ENOMEM, "host allocation failed");
   c->device = device;
   c->sm_count = prop.multiProcessorCount;
-  c->tuning = bmadgpu_tuning{256, 2, 1, 0, 0, {0, 0, 0}};
+  c->tuning = bmadgpu_tuning{256, 2, 1, 0, 0, {1, 0, 0}};  // shape by the particle count
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_err, sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&c->d_nwork, 2 * sizeof(int64_t)) != cudaSuccess) {
@@ -332,7 +332,6 @@ int bmadgpu_ctx_set_tuning(bmadgpu_ctx* c, const bmadgpu_tuning* t) {
     return fail(BMADGPU_EINVAL, "block must be 64, 128, 256 or 512");
   if (t->ctas_per_sm < 0 || t->turns_per_launch < 0) return fail(BMADGPU_EINVAL, "negative tuning value");
   c->tuning = *t;
-  c->tuned = true;
   return BMADGPU_OK;
 }
 
@@ -514,10 +513,13 @@ int bmadgpu_autotune(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_b
   t.beta = c->d_tbeta;
   t.state = c->d_tstate;
   const bmadgpu_tuning saved = c->tuning;
-  const bool was_tuned = c->tuned;
-  c->tuned = true;  // the trials' shapes are the candidates'
   struct Cand { int block, ctas, stage; };
-  static const Cand cands[] = {{128, 0, 0}, {128, 4, 0}, {128, 5, 0}, {128, 6, 0}, {256, 0, 0}, {256, 2, 0},
+#if defined(BG_TABLE_FORMS)
+  const Cand other = {64, 4, 0};   // a shape of the particle-count rule; 128 x 5 is 128 x 4 in this build
+#else
+  const Cand other = {128, 5, 0};
+#endif
+  const Cand cands[] = {{128, 0, 0}, {128, 4, 0}, other, {128, 6, 0}, {256, 0, 0}, {256, 2, 0},
                                {256, 3, 0}, {64, 8, 0},  {64, 12, 0}, {128, 0, 1}, {128, 4, 1}, {256, 2, 1}};
   cudaEvent_t e0, e1;
   CUDA_TRY(cudaEventCreate(&e0));
@@ -536,7 +538,6 @@ int bmadgpu_autotune(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_b
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     if (r) {
       c->tuning = saved;
-      c->tuned = was_tuned;
       return r;
     }
     CUDA_TRY(cudaEventSynchronize(e1));
@@ -548,7 +549,6 @@ int bmadgpu_autotune(bmadgpu_ctx* c, const bmadgpu_lattice* lat, const bmadgpu_b
     CUDA_TRY(cudaEventRecord(e1, c->stream));
     if (r) {
       c->tuning = saved;
-      c->tuned = was_tuned;
       return r;
     }
     CUDA_TRY(cudaEventSynchronize(e1));

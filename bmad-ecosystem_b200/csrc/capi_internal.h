@@ -51,7 +51,6 @@ struct bmadgpu_ctx {
   double* d_mom = nullptr;
   int64_t mom_cap = 0;
   int32_t* d_i32 = nullptr;       // state, ix_ele, ix_turn, location: 4 * cap
-  bool tuned = false;             // tuning was set by the caller or the autotuner
   bmadgpu_tuning tuning;
   int64_t launches = 0;           // kernel launches enqueued
   // scratch of the calls that need some for their own duration (Workspace), kept up to kKeptWork bytes

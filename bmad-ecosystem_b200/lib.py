@@ -175,12 +175,17 @@ class Context:
         t = Tuning()
         check(load().bmadgpu_ctx_get_tuning(self._h, C.byref(t)))
         return dict(block=t.block, ctas_per_sm=t.ctas_per_sm, stage_smem=t.stage_smem,
-                    turns_per_launch=t.turns_per_launch, compact=t.compact)
+                    turns_per_launch=t.turns_per_launch, compact=t.compact, automatic=t.reserved[0])
 
     def set_tuning(self, **kw):
+        """Changes the fields given. automatic=1 (a new context's) leaves the launch shape to the library's
+        rule on the particle count; giving block or ctas_per_sm pins them, unless automatic is given too."""
         cur = self.get_tuning()
+        if "block" in kw or "ctas_per_sm" in kw:
+            cur["automatic"] = 0
         cur.update(kw)
-        t = Tuning(cur["block"], cur["ctas_per_sm"], cur["stage_smem"], cur["turns_per_launch"], cur["compact"])
+        t = Tuning(cur["block"], cur["ctas_per_sm"], cur["stage_smem"], cur["turns_per_launch"], cur["compact"],
+                   (C.c_int32 * 3)(cur["automatic"], 0, 0))
         check(load().bmadgpu_ctx_set_tuning(self._h, C.byref(t)))
 
     @property

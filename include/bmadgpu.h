@@ -216,8 +216,10 @@ int bmadgpu_track1_bunch(bmadgpu_ctx* ctx, const bmadgpu_lattice* lat, bmadgpu_b
 int bmadgpu_ctx_synchronize(bmadgpu_ctx* ctx);
 
 /* Launch shape of the tracking kernel, chosen by the autotuner or set by the caller. A new
- * context starts with {256, 2, 1, 0, 0}, the fastest shape measured on both a 451- and a
- * 1801-element ring. */
+ * context starts with {256, 2, 1, 0, 0} and reserved[0] = 1: the shape goes by the particle count of
+ * each call, and block and ctas_per_sm are not used (libbmadgpu_cr.so has no such rule and launches
+ * them). reserved[0] = 0, which a structure filled in from zeros has, pins block and ctas_per_sm; any
+ * other field can be set without leaving the rule by changing it in what get_tuning returned. */
 typedef struct bmadgpu_tuning {
   int32_t block;              /* threads per CTA: 64, 128, 256 or 512 */
   int32_t ctas_per_sm;        /* minimum resident CTAs per SM the register budget is compiled for
@@ -227,7 +229,8 @@ typedef struct bmadgpu_tuning {
                                  when the copy leaves the resident CTAs per SM unchanged */
   int32_t turns_per_launch;   /* turns per kernel launch; 0 = all turns in one launch */
   int32_t compact;            /* compact the live-particle list between launches */
-  int32_t reserved[3];
+  int32_t reserved[3];        /* [0]: 1 = block and ctas_per_sm by the particle count, 0 = as given;
+                                 the others are not read */
 } bmadgpu_tuning;
 int bmadgpu_ctx_set_tuning(bmadgpu_ctx* ctx, const bmadgpu_tuning* tuning);
 int bmadgpu_ctx_get_tuning(const bmadgpu_ctx* ctx, bmadgpu_tuning* tuning);
