@@ -13,8 +13,10 @@
 //   k_adj_grad     one thread per (turn, particle): the reverse sweep with that cotangent, writing the
 //                  strength derivatives of the turn;
 //   k_adj_collect  adds them to each particle's [slot] column, last turn first.
-// Turns go through these in chunks from the last to the first, sized by kChunkBytes. No atomics and a
-// fixed order of every sum, so the result depends neither on scheduling nor on `every` or the chunks.
+// Turns go through these in chunks from the last to the first, sized by kChunkBytes; where the memory for
+// that is not there, in smaller chunks, from `every`-spaced checkpoints, and at last one turn of a part of
+// the particles (a slab) at a time (AdjPlan). No atomics and a fixed order of every sum, so the result
+// depends neither on scheduling nor on `every`, the chunks or the slabs.
 // k_adj_reduce: one CTA per slot sums the column in a fixed order (deterministic), divides by the
 // strength (scale form -> d/dk) and writes the gradient; slot n_slot sums the loss.
 
@@ -54,8 +56,9 @@ struct AdjArgs {
   double* beta;              // [N] in/out
   int32_t* state;            // [N] in/out
   double* turns;             // [rows][7][N]: states at turn starts
-  // a chunk of n_t turns: NT = n_t N threads, thread t N + j is particle j in turn row t of the chunk
-  int64_t NT;
+  // a chunk of n_t turns of the particles [j0, j0 + n_j): NT = n_t n_j threads, thread t n_j + q is particle
+  // j0 + q in turn row t of the chunk
+  int64_t NT, j0, n_j;
   double* inputs;            // [n_ele][7][NT]
   double* jac;               // [7][7][NT]: row c, the image of unit cotangent c
   double* lam_end;           // [7][NT]: cotangent at the end of the turn
@@ -146,7 +149,7 @@ template <bool REF>
 __global__ void __launch_bounds__(128) k_adj_inputs(const __grid_constant__ AdjArgs a, int row0, int first) {
   const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (i >= a.NT) return;
-  const int64_t t = i / a.N, j = i - t * a.N;
+  const int64_t t = i / a.n_j, j = a.j0 + i - t * a.n_j;
   if (a.state[j] != S_ALIVE) return;
   Particle p;
   get7(a.turns + (row0 + t) * 7 * a.N + j, a.N, p);
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(128) k_adj_inputs(const __grid_constant__ AdjA
 
 // The reverse sweep of one turn over its elements, cotangents a[NC]; GRAD: derivatives to part.
 template <int NC, bool GRAD>
-__device__ __forceinline__ void turn_sweep(const AdjArgs& A, int64_t i, Adj (&a)[NC]) {
+__device__ __forceinline__ void turn_sweep(const AdjArgs& A, int64_t i, int64_t j, Adj (&a)[NC]) {
   AdjCache k;
   double pz = 0, beta = 0;
   bool have = false;
@@ -187,21 +190,21 @@ __device__ __forceinline__ void turn_sweep(const AdjArgs& A, int64_t i, Adj (&a)
       const int slot = A.param_of_ele[ie];
       if (slot >= 0) {
         if (A.part) A.part[(int64_t)slot * A.NT + i] = gs[0];
-        else A.gradbuf[(int64_t)slot * A.N + i] += gs[0];
+        else A.gradbuf[(int64_t)slot * A.N + j] += gs[0];
       }
     }
   }
 }
 
 __global__ void __launch_bounds__(128) k_adj_turnjac(const __grid_constant__ AdjArgs A) {
-  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (i >= A.NT || A.state[i % A.N] != S_ALIVE) return;
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x, j = A.j0 + i % A.n_j;
+  if (i >= A.NT || A.state[j] != S_ALIVE) return;
   Adj a[7];
 #pragma unroll
   for (int c = 0; c < 7; c++)
     a[c] = Adj{c == 0 ? 1.0 : 0.0, c == 1 ? 1.0 : 0.0, c == 2 ? 1.0 : 0.0, c == 3 ? 1.0 : 0.0,
                c == 4 ? 1.0 : 0.0, c == 5 ? 1.0 : 0.0, c == 6 ? 1.0 : 0.0};
-  turn_sweep<7, false>(A, i, a);
+  turn_sweep<7, false>(A, i, j, a);
 #pragma unroll
   for (int c = 0; c < 7; c++) {
     double* q = A.jac + (int64_t)c * 7 * A.NT + i;
@@ -216,13 +219,13 @@ __global__ void __launch_bounds__(128) k_adj_turnjac(const __grid_constant__ Adj
 }
 
 __global__ void __launch_bounds__(kAdjBlock) k_adj_chain(const __grid_constant__ AdjArgs A, int n_t) {
-  const int64_t j = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x;
-  if (j >= A.N || A.state[j] != S_ALIVE) return;
+  const int64_t q = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x, j = A.j0 + q;
+  if (q >= A.n_j || A.state[j] != S_ALIVE) return;
   double l[7];
 #pragma unroll
   for (int k = 0; k < 7; k++) l[k] = A.lam[k * A.N + j];
   for (int t = n_t - 1; t >= 0; --t) {
-    const int64_t i = t * A.N + j;
+    const int64_t i = t * A.n_j + q;
     double m[49];
 #pragma unroll
     for (int k = 0; k < 49; k++) m[k] = A.jac[(int64_t)k * A.NT + i];
@@ -243,13 +246,14 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_chain(const __grid_constant__
 }
 
 __global__ void __launch_bounds__(128) k_adj_grad(const __grid_constant__ AdjArgs A) {
-  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  if (i >= A.NT || A.state[i % A.N] != S_ALIVE) return;
+  const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x, j = A.j0 + i % A.n_j;
+  if (i >= A.NT || A.state[j] != S_ALIVE) return;
   const double* q = A.lam_end + i;
   Adj a[1] = {Adj{q[0], q[A.NT], q[2 * A.NT], q[3 * A.NT], q[4 * A.NT], q[5 * A.NT], q[6 * A.NT]}};
-  turn_sweep<1, true>(A, i, a);
+  turn_sweep<1, true>(A, i, j, a);
 }
 
+// Of a chunk of several turns, which holds all particles (j0 = 0, n_j = N).
 __global__ void __launch_bounds__(128) k_adj_collect(const __grid_constant__ AdjArgs A, int n_t, int slot0) {
   const int64_t j = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (j >= A.N || A.state[j] != S_ALIVE) return;
@@ -292,6 +296,17 @@ cudaError_t adjoint_upload_constants() {
 }  // namespace bmadgpu
 
 namespace {
+
+// How the turns and particles of one call are divided. Turn starts: all of them where they fit (whole: one
+// segment of all turns), so that nothing is run twice; else the checkpoints of segments of `every` turns and,
+// after them, the turn starts of the segment in hand. chunk: turns of a chunk; slab: particles of a chunk of
+// one turn, all of them unless memory is short.
+struct AdjPlan {
+  bool whole;
+  int32_t seg, chunk;
+  int64_t slab;
+};
+constexpr int64_t kMinSlab = 32;
 
 // Device buffers of one call, carved from one block of the context's scratch.
 struct AdjBuffers {
@@ -360,43 +375,54 @@ extern "C" int bmadgpu_loss_grad(bmadgpu_ctx* c, const bmadgpu_lattice* lat, con
   }
   CUDA_TRY(cudaSetDevice(c->device));
   const int64_t N = b->n;
-  // Turn starts: all of them where they fit, so that nothing is run twice; else the checkpoints of the
-  // segments and, after them, the turn starts of the segment in hand.
-  const bool whole = (size_t)N * 56 * (size_t)n_turns <= kTurnStore;
-  const int32_t seg = whole ? n_turns : std::min(every, n_turns);
-  const int32_t n_seg = (n_turns + seg - 1) / seg;
   const size_t slots = (size_t)(n_param > 0 ? n_param : 1);
+  AdjPlan plan;
+  plan.whole = (size_t)N * 56 * (size_t)n_turns <= kTurnStore;
+  plan.seg = plan.whole ? n_turns : std::min(every, n_turns);
   const size_t per_turn = (size_t)N * 8 * ((size_t)n_ele * 7 + 49 + 7 + slots);
   // one wave of the Jacobian kernel (256 threads per SM), whose time a part of a second wave would double
   const size_t wave = std::max<size_t>(1, (size_t)c->sm_count * 256 / (size_t)N);
-  const int32_t chunk =
-      (int32_t)std::max<size_t>(1, std::min({kChunkBytes / per_turn, (size_t)seg, wave}));
-  const size_t CN = (size_t)chunk * N;
+  plan.chunk = (int32_t)std::max<size_t>(1, std::min({kChunkBytes / per_turn, (size_t)plan.seg, wave}));
+  plan.slab = N;
   double *d_vec, *d_beta, *d_turn, *d_ele, *d_jac, *d_lam_end, *d_part, *d_lam, *d_grad, *d_loss, *d_strength, *d_out;
   int32_t *d_state, *d_slot;
   Workspace work(c);
   AdjBuffers buf;
-  for (int pass = 0; pass < 2; pass++) {
+  auto lay_out = [&]() {
+    const size_t CN = (size_t)plan.chunk * (size_t)plan.slab;
+    const size_t n_seg = (size_t)((n_turns + plan.seg - 1) / plan.seg);
+    buf.used = 0;
     buf.get(&d_vec, 6 * N);
     buf.get(&d_beta, N);
     buf.get(&d_state, N);
-    buf.get(&d_turn, (size_t)(whole ? seg : n_seg + seg) * 7 * N);
+    buf.get(&d_turn, (plan.whole ? (size_t)plan.seg : n_seg + plan.seg) * 7 * N);
     buf.get(&d_ele, (size_t)n_ele * 7 * CN);
     buf.get(&d_jac, 49 * CN);
     buf.get(&d_lam_end, 7 * CN);
-    buf.get(&d_part, chunk > 1 ? slots * CN : 1);
+    buf.get(&d_part, plan.chunk > 1 ? slots * CN : 1);
     buf.get(&d_lam, 7 * (size_t)N);
     buf.get(&d_grad, slots * N);
     buf.get(&d_loss, N);
     buf.get(&d_strength, slots);
     buf.get(&d_out, slots + 1);
     buf.get(&d_slot, (size_t)n_ele);
-    if (pass == 0) {
-      if (!work.get(buf.used)) return fail(BMADGPU_ENOMEM, "cannot allocate the adjoint's device buffers");
-      buf.base = static_cast<unsigned char*>(work.ptr);
-      buf.used = 0;
+  };
+  for (lay_out(); !work.get(buf.used); lay_out()) {
+    if (plan.chunk > 1) {
+      plan.chunk /= 2;
+    } else if (plan.whole && (n_turns + every - 1) / every + every < n_turns) {
+      plan.whole = false;
+      plan.seg = every;
+    } else if (plan.slab > kMinSlab) {
+      plan.slab = std::max<int64_t>(kMinSlab, (plan.slab / 2 + 31) / 32 * 32);
+    } else {
+      return fail(BMADGPU_ENOMEM, "cannot allocate the adjoint's device buffers");
     }
   }
+  buf.base = static_cast<unsigned char*>(work.ptr);
+  lay_out();
+  const bool whole = plan.whole;
+  const int32_t seg = plan.seg, n_seg = (n_turns + seg - 1) / seg, chunk = plan.chunk;
   cudaStream_t s = c->stream;
   CUDA_TRY(cudaMemcpyAsync(d_vec, b->vec, 6 * N * sizeof(double), cudaMemcpyHostToDevice, s));
   CUDA_TRY(cudaMemcpyAsync(d_beta, b->beta, N * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -448,13 +474,16 @@ extern "C" int bmadgpu_loss_grad(bmadgpu_ctx* c, const bmadgpu_lattice* lat, con
     }
     for (int32_t end = nt; end > 0;) {
       const int32_t begin = std::max(0, end - chunk), n = end - begin;
-      a.NT = (int64_t)n * N;
-      const unsigned wide = (unsigned)((a.NT + 127) / 128);
-      inputs<<<wide, 128, 0, s>>>(a, row0 + begin, t0 + begin == 0);
-      k_adj_turnjac<<<wide, 128, 0, s>>>(a);
-      k_adj_chain<<<grid, kAdjBlock, 0, s>>>(a, n);
-      k_adj_grad<<<wide, 128, 0, s>>>(a);
-      c->launches += 4;
+      for (a.j0 = 0; a.j0 < N; a.j0 += plan.slab) {
+        a.n_j = std::min(plan.slab, N - a.j0);
+        a.NT = (int64_t)n * a.n_j;
+        const unsigned wide = (unsigned)((a.NT + 127) / 128);
+        inputs<<<wide, 128, 0, s>>>(a, row0 + begin, t0 + begin == 0);
+        k_adj_turnjac<<<wide, 128, 0, s>>>(a);
+        k_adj_chain<<<(unsigned)((a.n_j + kAdjBlock - 1) / kAdjBlock), kAdjBlock, 0, s>>>(a, n);
+        k_adj_grad<<<wide, 128, 0, s>>>(a);
+        c->launches += 4;
+      }
       for (int32_t s0 = 0; a.part && s0 < n_param; s0 += 32768) {
         const dim3 all((unsigned)((N + 127) / 128), (unsigned)std::min(n_param - s0, 32768));
         k_adj_collect<<<all, 128, 0, s>>>(a, n, s0);

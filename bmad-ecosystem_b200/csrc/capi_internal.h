@@ -56,6 +56,7 @@ struct bmadgpu_ctx {
   // scratch of the calls that need some for their own duration (Workspace), kept up to kKeptWork bytes
   void* d_work = nullptr;
   size_t work_cap = 0;
+  int64_t scratch_limit = 0;      // bmadgpu_selftest_scratch_limit
   // autotuner trial copies
   int64_t tune_cap = 0;
   double* d_tvec = nullptr;
@@ -64,8 +65,9 @@ struct bmadgpu_ctx {
 };
 
 // Device scratch for one call on a context: the context's own block, grown as needed and kept for the
-// next call (allocating and freeing 16 bytes a particle took longer than the statistics it served), or, above kKeptWork, a block freed with this object. A context is one host thread's and
-// its work is ordered by its stream; every user waits for its stream before it returns.
+// next call (allocating and freeing 16 bytes a particle took longer than the statistics it served), or, above
+// kKeptWork, a block freed with this object. A context is one host thread's and its work is ordered by its
+// stream; every user waits for its stream before it returns.
 constexpr size_t kKeptWork = (size_t)128 << 20;
 struct Workspace {
   bmadgpu_ctx* c;
@@ -77,9 +79,12 @@ struct Workspace {
   ~Workspace() {
     if (own) cudaFree(ptr);
   }
+  // False if there is no memory for it; a caller that can do with less may ask again.
   bool get(size_t bytes) {
+    if (c->scratch_limit > 0 && bytes > (size_t)c->scratch_limit) return false;
     if (bytes > kKeptWork) {
       own = cudaMalloc(&ptr, bytes) == cudaSuccess;
+      if (!own) cudaGetLastError();  // handled: not the next launch's error
       return own;
     }
     if (bytes > c->work_cap) {
@@ -87,6 +92,7 @@ struct Workspace {
       c->d_work = nullptr;
       c->work_cap = 0;
       if (cudaMalloc(&c->d_work, bytes) != cudaSuccess) {
+        cudaGetLastError();
         c->d_work = nullptr;
         return false;
       }

@@ -106,6 +106,13 @@ extern "C" int bmadgpu_cr_eval(bmadgpu_ctx* c, int32_t fn, const double* a, cons
   return BMADGPU_OK;
 }
 
+extern "C" int bmadgpu_selftest_scratch_limit(bmadgpu_ctx* c, int64_t bytes) {
+  if (!c) return fail(BMADGPU_EINVAL, "ctx is NULL");
+  if (bytes < 0) return fail(BMADGPU_EINVAL, "negative limit");
+  c->scratch_limit = bytes;
+  return BMADGPU_OK;
+}
+
 extern "C" int bmadgpu_selftest_division(bmadgpu_ctx* c, int64_t n, uint64_t seed, int64_t* mismatches) {
   if (!c || !mismatches || n < 0) return fail(BMADGPU_EINVAL, "bad argument");
   CUDA_TRY(cudaSetDevice(c->device));

@@ -259,6 +259,10 @@ int bmadgpu_measure_fp64_peak(bmadgpu_ctx* ctx, double* flops_per_s);
  * the device's a / b. 0 is the only correct answer. */
 int bmadgpu_selftest_division(bmadgpu_ctx* ctx, int64_t n, uint64_t seed, int64_t* mismatches);
 
+/* For tests of the calls that make do with less scratch (bmadgpu_loss_grad): this context's scratch
+ * requests above `bytes` fail as if the device had no more memory; 0 removes the limit. */
+int bmadgpu_selftest_scratch_limit(bmadgpu_ctx* ctx, int64_t bytes);
+
 /* The correctly rounded transcendentals the element maps use, evaluated on the device for n
  * arguments (device memory): fn 0 sin(a), 1 cos(a), 2 asin(a), 3 atan2(a, b), 4 sinh(a),
  * 5 cosh(a), 6 sincos(a) (sin in out[0, n), cos in out[n, 2n)), 7 sinhcosh(a) (likewise),
