@@ -50,8 +50,8 @@ struct BatchArgs {
   unsigned long long* n_out;         // [n_var] lengths of the compacted lists
   unsigned long long* queue;         // [2] work-item counters, zero at launch (the second for REF kernels)
   int32_t* err_flag;                 // bit 0: table staging wait timed out
-  uint32_t smem_bytes;               // dynamic shared memory for staging (0: read tables from global); set by
-                                     // batch_launch_track
+  uint32_t smem_bytes;               // dynamic shared memory for staging (0: read tables from global). To
+                                     // batch_launch_track: what the launch's tables need (default build)
   int32_t rare;                      // some variant's table has extra blocks / pitched offsets
   int32_t ref;                       // variants that track in the reference's order (Globals::hi_hot_pz = 0):
                                      // 0 none, 1 some, 2 all
@@ -72,7 +72,7 @@ struct BatchKernel {
   int block = 0, ppt = 1;
   const void* fn[3][2] = {};     // [BatchForm][with the frequency-map record path]
   int grid[3][2] = {};
-  uint32_t smem[3][2] = {};      // dynamic shared memory for staging tables
+  uint32_t smem[3][2] = {};      // shared memory for staging: the room for it (default build), else what is taken
 };
 
 cudaError_t batch_upload_constants();
@@ -85,8 +85,8 @@ cudaError_t batch_ref_rec_upload_constants();
 const void* batch_rec_kernel(int block, int minb, bool full = true);
 const void* batch_ref_kernel(int block, int minb, bool full);
 const void* batch_ref_rec_kernel(int block, int minb, bool full);
-// smem_bytes: shared memory for staging, as much as the largest table that may be staged. The default build
-// takes it for lattices in the reference's order alone, and no more than leaves the resident CTAs unchanged.
+// smem_bytes: shared memory for staging, as much as the largest table that may be staged; 0: none. The default
+// build stages lattices in the reference's order alone, tables up to what leaves the resident CTAs unchanged.
 cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_count, BatchKernel* out);
 // record: use the instantiation with the frequency-map record path (rounds with an FMA job). *launches: kernels
 // launched.

@@ -107,6 +107,7 @@ int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64
   a.err_flag = b->ctx->d_err;
   a.rare = b->rare;
   a.ref = b->ref;
+  a.smem_bytes = b->smem_bytes;
   for (int32_t c = 0; c < n_chunks; ++c) {
     const bool last = c == n_chunks - 1;
     a.turn_off = c * tpl;

@@ -384,6 +384,7 @@ void worker_main(bmadgpu_server* s) {
     std::vector<int64_t> round_jobs;
     bool round_records = false;
     int32_t round_rare = 0, round_ref = 0;  // round_ref: jobs of the round in the reference's order
+    uint32_t round_table = 0;               // their largest table that may be staged
     for (int32_t slot = 0; slot < (int32_t)s->slot_job.size(); ++slot) {
       const int64_t id = s->slot_job[slot];
       BatchVar& hv = s->h_vars[buf][slot];
@@ -404,7 +405,10 @@ void worker_main(bmadgpu_server* s) {
       j.last_round = r;
       round_jobs.push_back(id);
       round_records = round_records || j.fma;
-      round_ref += j.lat->G.hi_hot_pz == 0;
+      if (j.lat->G.hi_hot_pz == 0) {
+        round_ref++;
+        if (hv.table_bytes <= kServeStageBytes) round_table = std::max(round_table, hv.table_bytes);
+      }
     }
     const bool stopping = s->stop;
     lk.unlock();
@@ -450,6 +454,7 @@ void worker_main(bmadgpu_server* s) {
       a.queue = s->d_queue;
       a.err_flag = s->ctx->d_err;
       a.rare = round_rare;
+      a.smem_bytes = round_table;
       a.ref = round_ref == 0 ? 0 : round_ref < (int32_t)round_jobs.size() ? 1 : 2;
       int64_t launched = 0;
       Round rd;
