@@ -11,7 +11,8 @@
 // live list with a warp ballot and one atomic per warp, so compaction needs no extra pass.
 //
 // k_batch_plan: one CTA; exclusive scan of the tile counts (live count / tile, rounded up) over
-// the variants, reset of the work counter and of the next launch's live counts.
+// the variants (want 0 or 1: of those in the forms of fastmaps.cuh or in the reference's order, each with a
+// plan of its own in a launch of both), reset of the work counter and of the next launch's live counts.
 
 #include <cuda_runtime.h>
 
@@ -27,7 +28,7 @@ namespace bmadgpu {
 
 namespace {
 
-__global__ void k_batch_plan(const BatchVar* __restrict__ vars, int n_var, int tile, int turn_off, int identity,
+__global__ void k_batch_plan(const BatchVar* __restrict__ vars, int n_var, int tile, int turn_off, int identity, int want,
                              const unsigned long long* __restrict__ n_in, int64_t* __restrict__ tile_prefix,
                              unsigned long long* __restrict__ queue, unsigned long long* __restrict__ n_zero) {
   __shared__ long long warp_sums[32];
@@ -35,8 +36,7 @@ __global__ void k_batch_plan(const BatchVar* __restrict__ vars, int n_var, int t
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
   if (threadIdx.x == 0) {
     carry = 0;
-    queue[0] = 0;
-    queue[1] = 0;
+    *queue = 0;
   }
   __syncthreads();
   for (int base = 0; base < n_var; base += blockDim.x) {
@@ -44,7 +44,8 @@ __global__ void k_batch_plan(const BatchVar* __restrict__ vars, int n_var, int t
     long long tiles = 0;
     if (v < n_var) {
       const long long cnt = identity ? (long long)vars[v].n : (long long)n_in[v];
-      if (vars[v].n_turns > turn_off && cnt > 0) tiles = (cnt + tile - 1) / tile;
+      const bool mine = want < 0 || (vars[v].G.hi_hot_pz == 0) == (want != 0);
+      if (mine && vars[v].n_turns > turn_off && cnt > 0) tiles = (cnt + tile - 1) / tile;
       if (n_zero) n_zero[v] = 0;
     }
     long long x = tiles;  // inclusive scan within the warp
@@ -138,13 +139,13 @@ cudaError_t batch_upload_constants() {
   return cudaMemcpyToSymbol(c_cfull, cf, sizeof(cf));
 }
 
-cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_count, BatchKernel* out) {
+cudaError_t batch_resolve(const BatchLaunch& cfg, int ref, uint32_t smem_bytes, int sm_count, BatchKernel* out) {
   const Variant* v = pick(kVariants, cfg.block, cfg.ctas_per_sm);
   if (!v || cfg.particles_per_thread < 1) return cudaErrorInvalidValue;
   *out = BatchKernel();
   const void* fn[3][2];
 #if defined(BG_FAST_MAPS)
-  const Variant* m = pick(kRefShapes, cfg.block, cfg.ctas_per_sm);
+  const Variant* m = pick(kRefShapes, cfg.block, cfg.ref_ctas < 0 ? cfg.ctas_per_sm : cfg.ref_ctas);
   if (!m) return cudaErrorInvalidValue;
   fn[kBatchForms][0] = v->fn;
   fn[kBatchForms][1] = batch_rec_kernel(v->block, v->minb);
@@ -152,15 +153,16 @@ cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_co
     fn[form][0] = batch_ref_kernel(m->block, m->minb, form == kBatchFull);
     fn[form][1] = batch_ref_rec_kernel(m->block, m->minb, form == kBatchFull);
   }
-  const int first = kBatchForms;
+  const int first = ref < 2 ? kBatchForms : kBatchFull, last = ref > 0 ? kBatchLean : kBatchForms;
 #else
   for (int form : {kBatchFull, kBatchLean}) {
     fn[form][0] = form == kBatchFull ? v->fn : v->fn_lean;
     fn[form][1] = batch_rec_kernel(v->block, v->minb, form == kBatchFull);
   }
-  const int first = kBatchFull;
+  (void)ref;
+  const int first = kBatchFull, last = kBatchLean;
 #endif
-  for (int form = first; form <= kBatchLean; form++)
+  for (int form = first; form <= last; form++)
     for (int rec = 0; rec < 2; rec++) {
       const void* f = fn[form][rec];
       if (!f) return cudaErrorInvalidValue;
@@ -206,6 +208,7 @@ cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& args_in, c
 #endif
   for (int form : forms) {
     if (form < 0) continue;
+    if (!k.fn[form][record]) return cudaErrorInvalidValue;  // not resolved
 #if defined(BG_FAST_MAPS)
     // shared memory for a table that does not fit would only take it from L1 (4096 particles of a ring with
     // thin multipoles, 64 x 8: 5.3 ms against 3.3)
@@ -213,6 +216,10 @@ cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& args_in, c
 #else
     a.smem_bytes = k.smem[form][record];
 #endif
+    if (a.ref == 1 && form != kBatchForms) {  // the second plan (batch_launch_plan)
+      a.tile_prefix = args_in.tile_prefix + a.plan_stride;
+      a.queue = args_in.queue + 1;
+    }
     cudaError_t err = cudaLaunchKernel(k.fn[form][record], dim3((unsigned)k.grid[form][record]),
                                        dim3((unsigned)k.block), args, a.smem_bytes, stream);
     if (err != cudaSuccess) return err;
@@ -223,10 +230,19 @@ cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& args_in, c
 
 cudaError_t batch_launch_plan(const BatchVar* vars, int32_t n_var, int32_t tile, int32_t turn_off, bool identity,
                               const unsigned long long* n_in, int64_t* tile_prefix, unsigned long long* queue,
-                              unsigned long long* n_zero, cudaStream_t stream) {
-  k_batch_plan<<<1, 1024, 0, stream>>>(vars, n_var, tile, turn_off, identity ? 1 : 0, n_in, tile_prefix, queue,
-                                       n_zero);
-  return cudaGetLastError();
+                              unsigned long long* n_zero, int ref, int32_t plan_stride, cudaStream_t stream,
+                              int64_t* launches) {
+#if !defined(BG_FAST_MAPS)
+  ref = 0;
+#endif
+  for (int want = 0; want < (ref == 1 ? 2 : 1); want++) {
+    k_batch_plan<<<1, 1024, 0, stream>>>(vars, n_var, tile, turn_off, identity ? 1 : 0, ref == 1 ? want : -1, n_in,
+                                         tile_prefix + (int64_t)want * plan_stride, queue + want, n_zero);
+    cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+    (*launches)++;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t batch_launch_set_turns(BatchVar* vars, int32_t n_var, int32_t turn0, int32_t n_turns,

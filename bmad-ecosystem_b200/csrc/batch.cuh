@@ -48,19 +48,22 @@ struct BatchArgs {
   const unsigned long long* n_in;    // [n_var] live-list lengths (unused with live_in == nullptr)
   int32_t* live_out;                 // nullptr: no compaction after this launch
   unsigned long long* n_out;         // [n_var] lengths of the compacted lists
-  unsigned long long* queue;         // [2] work-item counters, zero at launch (the second for REF kernels)
+  unsigned long long* queue;         // work-item counter, zero at launch
   int32_t* err_flag;                 // bit 0: table staging wait timed out
   uint32_t smem_bytes;               // dynamic shared memory for staging (0: read tables from global). To
                                      // batch_launch_track: what the launch's tables need (default build)
   int32_t rare;                      // some variant's table has extra blocks / pitched offsets
   int32_t ref;                       // variants that track in the reference's order (Globals::hi_hot_pz = 0):
-                                     // 0 none, 1 some, 2 all
+                                     // 0 none, 1 some (tile_prefix and queue hold a second plan, for them),
+                                     // 2 all
+  int32_t plan_stride;               // from tile_prefix to the second plan's
 };
 
 struct BatchLaunch {
   int block = 128;
   int ctas_per_sm = 0;        // register budget selector, as LaunchCfg::ctas_per_sm
   int particles_per_thread = 1;
+  int ref_ctas = -1;          // the same for the kernels in the reference's order; -1: as ctas_per_sm
 };
 
 // Which instantiation a launch takes: the forms of fastmaps.cuh, or with the reference's element forms inline
@@ -85,19 +88,24 @@ cudaError_t batch_ref_rec_upload_constants();
 const void* batch_rec_kernel(int block, int minb, bool full = true);
 const void* batch_ref_kernel(int block, int minb, bool full);
 const void* batch_ref_rec_kernel(int block, int minb, bool full);
+// ref (as BatchArgs::ref): which sorts of lattice; a kernel that is not wanted is not loaded, since its stack
+// would widen every kernel's local memory (a served burst of small jobs took 4 % longer).
 // smem_bytes: shared memory for staging, as much as the largest table that may be staged; 0: none. The default
 // build stages lattices in the reference's order alone, tables up to what leaves the resident CTAs unchanged.
-cudaError_t batch_resolve(const BatchLaunch& cfg, uint32_t smem_bytes, int sm_count, BatchKernel* out);
+cudaError_t batch_resolve(const BatchLaunch& cfg, int ref, uint32_t smem_bytes, int sm_count, BatchKernel* out);
 // record: use the instantiation with the frequency-map record path (rounds with an FMA job). *launches: kernels
 // launched.
 cudaError_t batch_launch_track(const BatchKernel& k, const BatchArgs& a, cudaStream_t stream, bool record,
                                int64_t* launches);
 // Work plan for a launch: tile_prefix from the live counts (or the variants' sizes when
 // identity is set), restricted to variants with turns left after turn_off; zeroes the queue
-// counter and the next launch's counts (n_zero, nullable).
+// counter and the next launch's counts (n_zero, nullable). With variants of both sorts (ref 1) two plans: of those
+// in the forms of fastmaps.cuh to tile_prefix and queue[0], of those in the reference's order to
+// tile_prefix + plan_stride and queue[1].
 cudaError_t batch_launch_plan(const BatchVar* vars, int32_t n_var, int32_t tile, int32_t turn_off, bool identity,
                               const unsigned long long* n_in, int64_t* tile_prefix, unsigned long long* queue,
-                              unsigned long long* n_zero, cudaStream_t stream);
+                              unsigned long long* n_zero, int ref, int32_t plan_stride, cudaStream_t stream,
+                              int64_t* launches);
 // Sets turn0 and n_turns of every variant (the batch entry point's per-call values).
 cudaError_t batch_launch_set_turns(BatchVar* vars, int32_t n_var, int32_t turn0, int32_t n_turns,
                                    cudaStream_t stream);

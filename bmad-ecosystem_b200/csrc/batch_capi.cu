@@ -77,7 +77,7 @@ int resolve(bmadgpu_batch* b, BatchKernel* k) {
   cfg.block = tu.block;
   cfg.ctas_per_sm = tu.ctas_per_sm;
   cfg.particles_per_thread = tu.particles_per_thread;
-  CUDA_TRY(batch_resolve(cfg, tu.stage_smem ? b->smem_bytes : 0, b->ctx->sm_count, k));
+  CUDA_TRY(batch_resolve(cfg, b->ref, tu.stage_smem ? b->smem_bytes : 0, b->ctx->sm_count, k));
   return BMADGPU_OK;
 }
 
@@ -88,8 +88,8 @@ int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64
   const int32_t tpl = tu.turns_per_launch > 0 ? std::min(tu.turns_per_launch, n_turns) : n_turns;
   const int32_t n_chunks = (n_turns + tpl - 1) / tpl;
   cudaStream_t s = b->ctx->stream;
-  CUDA_TRY(batch_launch_plan(b->d_vars, b->n_var, tile, 0, true, nullptr, b->d_prefix, b->d_queue, b->d_cnt, s));
-  (*launches)++;
+  CUDA_TRY(batch_launch_plan(b->d_vars, b->n_var, tile, 0, true, nullptr, b->d_prefix, b->d_queue, b->d_cnt, b->ref,
+                             b->n_var + 1, s, launches));
   BatchArgs a;
   std::memset(&a, 0, sizeof(a));
   a.vars = b->d_vars;
@@ -107,6 +107,7 @@ int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64
   a.err_flag = b->ctx->d_err;
   a.rare = b->rare;
   a.ref = b->ref;
+  a.plan_stride = b->n_var + 1;
   a.smem_bytes = b->smem_bytes;
   for (int32_t c = 0; c < n_chunks; ++c) {
     const bool last = c == n_chunks - 1;
@@ -119,8 +120,7 @@ int enqueue_calls(bmadgpu_batch* b, const BatchKernel& k, int32_t n_turns, int64
     CUDA_TRY(batch_launch_track(k, a, s, false, launches));
     if (!last) {
       CUDA_TRY(batch_launch_plan(b->d_vars, b->n_var, tile, (c + 1) * tpl, false, a.n_out, b->d_prefix, b->d_queue,
-                                 b->d_cnt + (size_t)((c + 1) & 1) * b->n_var, s));
-      (*launches)++;
+                                 b->d_cnt + (size_t)((c + 1) & 1) * b->n_var, b->ref, b->n_var + 1, s, launches));
     }
   }
   return BMADGPU_OK;
@@ -263,7 +263,7 @@ int bmadgpu_batch_create(bmadgpu_ctx* c, int32_t n_var, const bmadgpu_lattice* c
       cudaMalloc(&b->d_live[0], T * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_live[1], T * sizeof(int32_t)) != cudaSuccess ||
       cudaMalloc(&b->d_cnt, 2 * sizeof(unsigned long long) * n_var) != cudaSuccess ||
-      cudaMalloc(&b->d_prefix, sizeof(int64_t) * (n_var + 1)) != cudaSuccess ||
+      cudaMalloc(&b->d_prefix, 2 * sizeof(int64_t) * (n_var + 1)) != cudaSuccess ||
       cudaMalloc(&b->d_queue, 2 * sizeof(unsigned long long)) != cudaSuccess) {
     bmadgpu_batch_destroy(b);
     return fail(BMADGPU_ENOMEM, "cannot allocate the batch's device state");

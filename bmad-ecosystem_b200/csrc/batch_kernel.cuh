@@ -43,8 +43,8 @@ __device__ __noinline__ void fma_record(const BatchVar& v, int64_t j, int32_t t_
 // REC = false code, which has no record path at all. REF (default build): the reference's element order inline,
 // for the lattices that track in it (Globals::hi_hot_pz = 0), where with the forms of fastmaps.cuh each of
 // their elements is an out-of-line call (4096 particles of a ring with thin multipoles between its elements,
-// 4 turns: 10.6 ms against 6.4). A launch that holds lattices of both sorts is one of each kernel, which
-// leave each other's work items alone (a.ref == 1).
+// 4 turns: 10.6 ms against 6.4). A launch that holds lattices of both sorts is one of each kernel, each with a
+// plan of its own work items.
 template <int BLOCK, int MINB, bool REC, bool FULL = true, bool REF = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_constant__ BatchArgs a, int ppt) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -70,12 +70,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
 
   for (;;) {
     if (threadIdx.x == 0) {
-      long long item;
-      int v;
-      for (;;) {
-        item = (long long)atomicAdd(a.queue + REF, 1ull);
-        v = -1;
-        if (item >= total) break;
+      const long long item = (long long)atomicAdd(a.queue, 1ull);
+      int v = -1;
+      if (item < total) {
         // last variant whose first item is <= item (variants without items share their
         // successor's prefix value and are skipped)
         int lo = 0, hi = a.n_var - 1;
@@ -85,7 +82,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_batch_track(const __grid_consta
           else hi = mid - 1;
         }
         v = lo;
-        if (a.ref != 1 || (a.vars[v].G.hi_hot_pz == 0) == REF) break;
       }
       s_item = item;
       s_var = v;

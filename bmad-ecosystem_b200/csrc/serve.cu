@@ -160,7 +160,9 @@ struct bmadgpu_server {
   // pinned mirrors, one per round in flight
   BatchVar* h_vars[kRoundsInFlight] = {nullptr, nullptr};
   unsigned long long* h_cnt[kRoundsInFlight] = {nullptr, nullptr};
-  BatchKernel kern;
+  BatchLaunch shape;
+  BatchKernel kern;              // the reference order's kernels from the first round that wants them
+  bool kern_ref = false;
   // record arena for frequency-map jobs (doubles)
   double* d_rec = nullptr;
   int64_t rec_capacity = 0;
@@ -455,19 +457,25 @@ void worker_main(bmadgpu_server* s) {
       a.err_flag = s->ctx->d_err;
       a.rare = round_rare;
       a.smem_bytes = round_table;
+      a.plan_stride = s->cfg.max_jobs + 1;
       a.ref = round_ref == 0 ? 0 : round_ref < (int32_t)round_jobs.size() ? 1 : 2;
       int64_t launched = 0;
+      if (round_ref && !s->kern_ref) {
+        ok = batch_resolve(s->shape, 1, s->cfg.stage_smem ? kServeStageBytes : 0, s->ctx->sm_count, &s->kern) ==
+             cudaSuccess;
+        s->kern_ref = ok;
+      }
       Round rd;
       rd.index = r;
       rd.parity = parity;
       rd.jobs = round_jobs;
       rd.done = nullptr;
-      ok = cudaEventCreate(&rd.t0) == cudaSuccess && cudaEventCreate(&rd.t1) == cudaSuccess &&
+      ok = ok && cudaEventCreate(&rd.t0) == cudaSuccess && cudaEventCreate(&rd.t1) == cudaSuccess &&
            cudaEventRecord(rd.t0, c) == cudaSuccess &&
            cudaMemcpyAsync(s->d_vars, s->h_vars[buf], sizeof(BatchVar) * n_var, cudaMemcpyHostToDevice, c) ==
                cudaSuccess &&
-           batch_launch_plan(s->d_vars, n_var, a.tile, 0, false, a.n_in, s->d_prefix, s->d_queue, a.n_out, c) ==
-               cudaSuccess &&
+           batch_launch_plan(s->d_vars, n_var, a.tile, 0, false, a.n_in, s->d_prefix, s->d_queue, a.n_out, a.ref,
+                             a.plan_stride, c, &launched) == cudaSuccess &&
            batch_launch_track(s->kern, a, c, round_records, &launched) == cudaSuccess &&
            cudaMemcpyAsync(s->h_cnt[buf], a.n_out, sizeof(unsigned long long) * n_var, cudaMemcpyDeviceToHost, c) ==
                cudaSuccess &&
@@ -631,11 +639,18 @@ int bmadgpu_server_create(bmadgpu_ctx* c, const bmadgpu_server_config* cfg_in, b
   if (cfg.max_jobs == 0) cfg.max_jobs = 4096;
   if (cfg.element_steps == 0) cfg.element_steps = 4096;
   if (cfg.target_live == 0) cfg.target_live = 1 << 20;
+  int ref_ctas = -1;
   if (cfg.block == 0) {
+    // The reference's order wants 128 x 3 (168 registers): electric multipoles, thin multipoles or cavities
+    // in a ring, 16,384 particles, 2 turns 14.1, 2.9 and 5.4 ms against 16.0 to 17.2, 3.3 and 6.3 with 128 x 4;
+    // 98,304 particles 27.9, 5.8 and 10.8 against 30.0, 6.4 and 11.5. For the others
     // 128 x 4 measured fastest on the mixed request stream (200 jobs: 1.59e7 particle-turns/s
     // against 1.45e7 for 64 x 12 and 1.57e7 for 256 x 2)
     cfg.block = 128;
-    if (cfg.ctas_per_sm == 0) cfg.ctas_per_sm = 4;
+    if (cfg.ctas_per_sm == 0) {
+      cfg.ctas_per_sm = 4;
+      ref_ctas = 3;
+    }
   }
   CUDA_TRY(cudaSetDevice(c->device));
   size_t free_b = 0, total_b = 0;
@@ -663,7 +678,7 @@ int bmadgpu_server_create(bmadgpu_ctx* c, const bmadgpu_server_config* cfg_in, b
             cudaMalloc(&s->d_live[1], C * sizeof(int32_t)) == cudaSuccess &&
             cudaMalloc(&s->d_vars, J * sizeof(BatchVar)) == cudaSuccess &&
             cudaMalloc(&s->d_cnt, 2 * J * sizeof(unsigned long long)) == cudaSuccess &&
-            cudaMalloc(&s->d_prefix, (J + 1) * sizeof(int64_t)) == cudaSuccess &&
+            cudaMalloc(&s->d_prefix, 2 * (J + 1) * sizeof(int64_t)) == cudaSuccess &&
             cudaMalloc(&s->d_queue, 2 * sizeof(unsigned long long)) == cudaSuccess;
   for (int i = 0; ok && i < kRoundsInFlight; ++i)
     ok = cudaHostAlloc(&s->h_vars[i], J * sizeof(BatchVar), cudaHostAllocPortable) == cudaSuccess &&
@@ -684,11 +699,12 @@ int bmadgpu_server_create(bmadgpu_ctx* c, const bmadgpu_server_config* cfg_in, b
     }
   }
   if (ok) {
-    BatchLaunch bl;
+    BatchLaunch& bl = s->shape;
     bl.block = cfg.block;
     bl.ctas_per_sm = cfg.ctas_per_sm;
     bl.particles_per_thread = 1;
-    ok = batch_resolve(bl, cfg.stage_smem ? kServeStageBytes : 0, c->sm_count, &s->kern) == cudaSuccess;
+    bl.ref_ctas = ref_ctas;
+    ok = batch_resolve(bl, 0, cfg.stage_smem ? kServeStageBytes : 0, c->sm_count, &s->kern) == cudaSuccess;
   }
   if (!ok) {
     bmadgpu_server_destroy(s);

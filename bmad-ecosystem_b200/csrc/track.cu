@@ -234,8 +234,8 @@ static const Variant kVariants[] = {
 // CTAs per SM every warp has a scheduler nearly to itself and only its own latency counts: the
 // register budget without spills, and small CTAs so that all SMs get some (10,000 particles, 50-cell
 // ring: 0.16 ms a turn against 0.20 with 80 registers). A bunch that fills the chip wants the warps:
-// 24 per SM at 80 registers (1M particles, 200-cell ring: 16.4 ms a turn against 19.9 with 16 warps at
-// 128 registers and 27.2 with 8 at 255). The reference's element order needs more registers: 256 x 2 there.
+// 24 per SM at 80 registers (1M particles, 200-cell ring: 17.3 ms a turn; in one sweep of shapes 16.4
+// against 19.9 with 16 warps at 128 registers and 27.2 with 8 at 255). The reference's element order needs more registers: 256 x 2 there.
 static void shape_for(int64_t n, int sm_count, bool ref, LaunchCfg* cfg) {
   const int64_t row = (int64_t)64 * sm_count;  // one 64-thread CTA on every SM
   if (ref) {

@@ -288,8 +288,10 @@ int64_t bmadgpu_sizeof(int32_t which); /* 0 element, 1 param, 2 bunch, 3 tuning,
  * all of them: one structure-of-arrays block per variant, laid out one after another
  * (vec: variant v's [6][n_v] block follows variant v-1's; beta, t, state, ix_ele, ix_turn and
  * location likewise). Each launch hands out work items -- (variant, tile of live particles) --
- * from a device counter; CTAs stage the item's element table in shared memory when the variant
- * changes. Between launches the surviving particles of each variant are compacted (fused in the
+ * from a device counter. libbmadgpu.so reads the element tables through L1, except those of lattices
+ * that track in the reference's element order (more than a third of their elements without a faster
+ * form), which its CTAs stage in shared memory when the variant changes, where there is room beside
+ * the resident CTAs; libbmadgpu_cr.so stages every table that fits. Between launches the surviving particles of each variant are compacted (fused in the
  * tracking kernel: warp ballot + one atomic per warp). The launch sequence of a call is captured
  * once into a CUDA graph and replayed. Results per particle are bit-identical to
  * bmadgpu_track_bunch_device on the same variant with the same turns_per_launch. */
@@ -300,7 +302,8 @@ typedef struct bmadgpu_batch_tuning {
   int32_t ctas_per_sm;          /* register budget as in bmadgpu_tuning (0 = most registers) */
   int32_t particles_per_thread; /* particles a thread tracks per work item: tile = block x this */
   int32_t turns_per_launch;     /* turns per launch, compaction in between; 0 = one launch */
-  int32_t stage_smem;           /* stage each variant's element table in shared memory */
+  int32_t stage_smem;           /* stage element tables in shared memory (which: see above); the
+                                   autotuner tries both settings where some table may be staged */
   int32_t use_graph;            /* replay each call's launch sequence as a CUDA graph */
   int32_t reserved[2];
 } bmadgpu_batch_tuning;
@@ -358,8 +361,8 @@ typedef struct bmadgpu_server_config {
   int64_t target_live;     /* no admission while this many live particles are resident (0: 1,048,576) */
   int32_t policy;          /* BMADGPU_SERVE_SRPT or BMADGPU_SERVE_FIFO */
   int32_t block;           /* round kernel shape as bmadgpu_batch_tuning (0: 128) */
-  int32_t ctas_per_sm;     /* (0 with block 0: 4) */
-  int32_t stage_smem;      /* stage element tables of up to 64 KiB in shared memory */
+  int32_t ctas_per_sm;     /* (0 with block 0: 4, and 3 for lattices in the reference's element order) */
+  int32_t stage_smem;      /* stage element tables of up to 64 KiB in shared memory (as in a batch) */
   int32_t record_mib;      /* record arena of frequency-map jobs in MiB (0: a quarter of the device
                               memory still free after the particle arena) */
   int32_t reserved[3];
@@ -420,8 +423,11 @@ int bmadgpu_server_get_stats(bmadgpu_server* server, bmadgpu_server_stats* stats
  * d(loss)/d(k) for element param_ele[i] (0-based): k1 of a quadrupole, k2 of a sextupole, k3 of
  * an octupole; the element's strength must be non-zero and its other field coefficients must scale
  * with it (no hkick/vkick; multipoles only with scale_multipoles). Computed by a hand-written
- * adjoint of the element maps, one thread per particle, with a checkpoint every checkpoint_every
- * turns and recomputation in between. Lattices with edge fringe, bends with k1 or multipoles,
+ * adjoint of the element maps, with a thread per turn and particle where turns need not follow one
+ * another. It keeps the state at the start of every turn while that takes up to 1 GiB, else (or where
+ * the memory is short) checkpoints every checkpoint_every turns with recomputation in between; up to
+ * 2 GiB more hold a stretch of turns in hand, less where the device has less. The result depends on
+ * none of this. Lattices with edge fringe, bends with k1 or multipoles,
  * thin multipoles, pitched or offset bends, electric multipoles or elements of more than 16 steps
  * give BMADGPU_EUNSUPPORTED. Lost particles
  * leave the loss (the set of survivors is held fixed). */
