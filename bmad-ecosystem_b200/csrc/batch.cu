@@ -147,6 +147,11 @@ cudaError_t batch_resolve(const BatchLaunch& cfg, int ref, uint32_t smem_bytes, 
 #if defined(BG_FAST_MAPS)
   const Variant* m = pick(kRefShapes, cfg.block, cfg.ref_ctas < 0 ? cfg.ctas_per_sm : cfg.ref_ctas);
   if (!m) return cudaErrorInvalidValue;
+  if (ref > 0) {
+    cudaError_t err = batch_ref_upload_constants();
+    if (err != cudaSuccess) return err;
+    if ((err = batch_ref_rec_upload_constants()) != cudaSuccess) return err;
+  }
   fn[kBatchForms][0] = v->fn;
   fn[kBatchForms][1] = batch_rec_kernel(v->block, v->minb);
   for (int form : {kBatchFull, kBatchLean}) {

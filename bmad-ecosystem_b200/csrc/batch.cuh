@@ -79,7 +79,8 @@ struct BatchKernel {
 };
 
 cudaError_t batch_upload_constants();
-// The other translation units' copies of the tables, and their instantiations of a shape: with the record
+// The other translation units' copies of the tables (those of the reference's order filled by batch_resolve,
+// so that a context loads them only when it wants them), and their instantiations of a shape: with the record
 // path (full: every element form, else the lean one), in the reference's order (default build; shapes of
 // BG_REF_SHAPES, else null), and with both.
 cudaError_t batch_rec_upload_constants();

@@ -189,10 +189,6 @@ cudaError_t upload_constants() {
   if (e != cudaSuccess) return e;
   e = batch_rec_upload_constants();
   if (e != cudaSuccess) return e;
-  e = batch_ref_upload_constants();
-  if (e != cudaSuccess) return e;
-  e = batch_ref_rec_upload_constants();
-  if (e != cudaSuccess) return e;
   return adjoint_upload_constants();
 }
 
