@@ -439,8 +439,8 @@ int bmadgpu_batch_autotune(bmadgpu_batch* b, int32_t sample_turns, bmadgpu_batch
   struct Shape {
     int block, ctas;
   };
-  static const Shape shapes[] = {{128, 0}, {128, 4}, {128, 5}, {128, 6}, {256, 0},
-                                 {256, 2}, {256, 3}, {64, 8},  {64, 12}, {512, 1}};
+  static const Shape shapes[] = {{128, 0}, {128, 4}, {128, 5}, {128, 6}, {256, 0}, {256, 2},
+                                 {256, 3}, {64, 4},  {64, 8},  {64, 12}, {512, 1}};
   for (int stage = 1; stage >= 0 && !r; --stage) {
     if (stage && b->smem_bytes == 0) continue;
     for (const Shape& sh : shapes) {
