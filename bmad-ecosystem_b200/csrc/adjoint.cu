@@ -224,13 +224,16 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_chain(const __grid_constant__
   double l[7];
 #pragma unroll
   for (int k = 0; k < 7; k++) l[k] = A.lam[k * A.N + j];
+  const int64_t NT = A.NT, n_j = A.n_j;
+  const double* __restrict__ jac = A.jac + q;
+  double* __restrict__ lam_end = A.lam_end + q;
   for (int t = n_t - 1; t >= 0; --t) {
-    const int64_t i = t * A.n_j + q;
+    const int64_t i = t * n_j;
     double m[49];
 #pragma unroll
-    for (int k = 0; k < 49; k++) m[k] = A.jac[(int64_t)k * A.NT + i];
+    for (int k = 0; k < 49; k++) m[k] = jac[(int64_t)k * NT + i];
 #pragma unroll
-    for (int k = 0; k < 7; k++) A.lam_end[k * A.NT + i] = l[k];
+    for (int k = 0; k < 7; k++) lam_end[k * NT + i] = l[k];
     double s[7];
 #pragma unroll
     for (int k = 0; k < 7; k++) {

@@ -1090,6 +1090,7 @@ int pack_lattice(const bmadgpu_element* eles, int n_ele, const bmadgpu_param& p,
           double angle = g * step_len;
           eblk = extra_block(e, p, ae, be, ix_elec_max, step_len * 0.5, step_len * 1.0);
           double gl = g * step_len;
+          if (!(step_len > 0) || !(std::fabs(gl) <= 1)) flags |= F_BEND_LONG;
           blk = {step_len, g, g_tot, dg, angle, l_cos(angle), l_sin(angle), sinc0(angle), cosc0(angle),
                  (gl * gl) * sincc0(angle), (b1 != 0 && e.l != 0) ? b1 / e.l : 0.0,
                  r_step * p.p0c / (2.99792458e8 * p.charge)};

@@ -36,6 +36,7 @@ enum Flag : uint16_t {
   F_BEND_K1 = 1 << 7,      // sbend body with k1 (sbend_body_with_k1_map)
   F_REF_ORB_N0 = 1 << 8,   // thin multipole: n = 0 as a zero-length bend (MAD convention)
   F_BEND_DRIFT = 1 << 9,   // sbend with g == 0 and dg == 0 or zero step: drift body
+  F_BEND_LONG = 1 << 10,   // sbend body step of no positive length or of more than a radian (adjoint.cuh)
   F_TILT = 1 << 11,        // misalign block carries a non-zero tilt rotation
   F_KICK_B_FROM2 = 1 << 12, // both kick arrays: every a_n zero and b_0 = b_1 = 0, at least 3 orders
   F_PITCH = 1 << 13,       // misalign block of the pitched form (straight elements) or the bend frame
