@@ -5,7 +5,8 @@
 // items of variant v are numbered tile_prefix[v] .. tile_prefix[v+1]-1. A CTA that moves to a
 // new variant takes up that variant's element table: the element forms of the default build read it from
 // global memory through L1; the correctly rounded build, and lattices in the reference's order, re-stage it
-// into shared memory with a bulk copy (mbarrier completion, bounded wait, the phase bit flipping on every use). Each thread tracks
+// into shared memory with a bulk copy (mbarrier completion, bounded wait, the phase bit flipping on every
+// use). Each thread tracks
 // `ppt` particles of the tile one after another, each through all turns of the launch, with the
 // same per-particle code as k_track (particle.cuh). Survivors are appended to the variant's next
 // live list with a warp ballot and one atomic per warp, so compaction needs no extra pass.

@@ -1,5 +1,6 @@
 // batch_ref.cu -- the instantiations of k_batch_track with the reference's element order inline
-// (batch_kernel.cuh, REF), for lattices without forms in fastmaps.cuh for many of their elements. The correctly rounded build tracks everything in that order and has none.
+// (batch_kernel.cuh, REF), for lattices without forms in fastmaps.cuh for many of their elements. The correctly
+// rounded build tracks everything in that order and has none.
 
 #include <cuda_runtime.h>
 

@@ -182,7 +182,8 @@ int check_err_flag(bmadgpu_ctx* c) {
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (h) {
     cudaMemsetAsync(c->d_err, 0, sizeof(int32_t), c->stream);
-    return fail(BMADGPU_ETIMEDOUT, "element-table staging wait timed out (the results are correct: the table was read or copied from global memory)");
+    return fail(BMADGPU_ETIMEDOUT, "element-table staging wait timed out (the results are correct: the table was read "
+                                   "or copied from global memory)");
   }
   return BMADGPU_OK;
 }
